@@ -86,7 +86,7 @@ k_adj_drift_paint(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
     const float ke = rec ? cf[a.it * 3 + 2] : 0.f;
     const float dr = rec ? cf[a.it * 3 + 1] : 0.f;
     const float* lr = a.lrho + S.m_off;
-    float* m = a.rho + S.m_off;
+    float* m = a.rho + S.r_off;
     const bool ck = rec && a.ckpt && (a.it % a.ckpt_every == 0);
     const float* ckd =
         ck ? a.ckpt + (int64_t)(a.it / a.ckpt_every) * 2 * a.total_np * 3
@@ -129,8 +129,8 @@ k_adj_drift_paint(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
       if (a.it < 0) continue;
       const float3 x = mesh_pos(S, i, j, k, d);
       if (!finite3(x.x, x.y, x.z)) atomicOr(a.status, FPM_STATUS_NONFINITE_POS);
-      paint8(m, S.mx, S.my, S.mz, cic_axis(x.x, S.mx), cic_axis(x.y, S.my),
-             cic_axis(x.z, S.mz));
+      paint8(m, S.pairs, cic8(cic_axis(x.x, S.mx), cic_axis(x.y, S.my),
+                              cic_axis(x.z, S.mz), S.my, S.mz));
     }
   }
 }

@@ -23,32 +23,6 @@
 // checkpoints, intermediate states) are written through the carried index.
 #include "fpm_bin.cuh"
 
-// Lanes of k_step_sorted that deposit into the same base cell sum their
-// weights with a segmented shuffle reduction and deposit once (1), or each
-// lane deposits its own (0).
-#ifndef FPM_SORTED_SEGSUM
-#define FPM_SORTED_SEGSUM 1
-#endif
-// Runs of k_step_sorted whose base cells are z-adjacent merge the four
-// deposits they share (1), or each deposits its eight (0).  Measured on
-// B200 (re-sorted every 16 steps; step kernels per 40-step simulation):
-// 3.09 against 3.01 ms at 128^3, 21.4 against 20.7 ms at 256^3 -- the
-// shuffles cost more than the reductions they save.
-#ifndef FPM_SORTED_ZMERGE
-#define FPM_SORTED_ZMERGE 0
-#endif
-// k_step_sorted paints through a shared-memory box of cells around its
-// chunk (1) or straight into the density (0).  Measured on B200 (particles
-// re-sorted every 16 steps; step kernels per 40-step simulation): 4.12 ms
-// with the box against 2.99 ms without at 128^3, 28.9 against 20.7 ms at
-// 256^3 -- the shared-memory atomics, the barriers and the flush of each
-// chunk cost more than the L2 reductions they save, once runs of lanes in
-// one cell already deposit once (the segmented sums; without them the
-// step takes 3.46 ms at 128^3).
-#ifndef FPM_SORTED_BOX
-#define FPM_SORTED_BOX 0
-#endif
-
 namespace fpm {
 
 namespace {
@@ -354,16 +328,6 @@ __device__ __forceinline__ int rel_cell(int c, int o, int m) {
   return r + T / 2;
 }
 
-// Offset of periodic cell c from a box origin o on an axis of m cells: the
-// representative of c - o (mod m) in (-m/2, m/2], so a box no larger than
-// the mesh sees every cell at most once; the caller tests 0 <= r < size.
-__device__ __forceinline__ int box_rel(int c, int o, int m) {
-  int r = c - o;
-  if (r > (m >> 1)) r -= m;
-  else if (r <= -(m >> 1)) r += m;
-  return r;
-}
-
 // The binned leapfrog step: one tile of T^3 force-mesh cells per block
 // iteration.  Per particle the arithmetic is k_step's (readout, closing
 // kick, opening kick, drift, paint), in the same order and rounding.  The
@@ -393,7 +357,7 @@ k_step_binned(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
     const float fac = a.ffac[s];
     const float invb = 1.0f / (float)S.bf;
     const int64_t mcells = (int64_t)S.mx * S.my * S.mz;
-    float* m = a.rho + S.m_off;
+    float* m = a.rho + S.r_off;
     const unsigned t = (unsigned)(ch - S.ch_t);
     const unsigned r = t / (unsigned)S.ntz;
     const int oz = (int)(t - r * (unsigned)S.ntz) * T;
@@ -470,7 +434,7 @@ k_step_binned(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
           atomicAdd(tq + 1, __fmul_rn(c1.wxy[q], c1.wz1));
         }
       } else {
-        paint_cic8(m, c1, 1.f);
+        paint8(m, S.pairs, c1);
       }
     }
     if (last) continue;
@@ -482,7 +446,13 @@ k_step_binned(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
       const int cy = wrap_near(oy - 1 + row % RX, S.my);
       const int cx = wrap_near(ox - 1 + row / RX, S.mx);
       const int cz = wrap_near(oz - 4 + 4 * zg, S.mz);
-      red_add_f4(m + ((int64_t)cx * S.my + cy) * S.mz + cz, v);
+      const int64_t c = ((int64_t)cx * S.my + cy) * S.mz + cz;
+      if (S.pairs) {  // whole-cell sums: the lower halves of four z pairs
+        red_add_f4(m + 2 * c, make_float4(v.x, 0.f, v.y, 0.f));
+        red_add_f4(m + 2 * c + 4, make_float4(v.z, 0.f, v.w, 0.f));
+      } else {
+        red_add_f4(m + c, v);
+      }
     }
     __syncthreads();  // the next tile zeroes the shared copy
   }
@@ -499,19 +469,9 @@ k_step_binned(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
 // (5 steps) and only the run's first lane issues the reductions.  The sums
 // of a run are formed in a different order than one deposit at a time
 // (FP32 rounding, as any order of the reference's scatter).
-template <bool BOX>
 __global__ void __launch_bounds__(kThreads, FPM_STEP_MINBLOCKS)
 k_step_sorted(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
               int64_t nchunks, BinStepArgs b) {
-  // BOX: the paint goes into a shared-memory box of cells around the
-  // chunk (BX x-planes from the first particle's cell less two, and the
-  // y and z extent of its 16^3 tile with a margin: z from four before, so
-  // the box flushes as aligned float4), then into rho with one 16-byte
-  // vector reduction per non-zero group of four; deposits outside the box
-  // go to rho directly.
-  constexpr int BX = 8, BY = 20, BZ = 24, BN = BX * BY * BZ;
-  __shared__ __align__(16) float box[BOX ? BN : 4];
-  __shared__ int box_org[3];
   pdl_wait();  // the force meshes of the solve before
   const StepArgs& a = b.a;
   const int lane = threadIdx.x & 31;
@@ -528,30 +488,9 @@ k_step_sorted(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
     const float fac = a.ffac[s];
     const float invb = 1.0f / (float)S.bf;
     const int64_t mcells = (int64_t)S.mx * S.my * S.mz;
-    float* m = a.rho + S.m_off;
+    float* m = a.rho + S.r_off;
     const int64_t first = S.p_off + (ch - S.ch_p) * kChunk;
     const int64_t end = S.p_off + S.np;
-    int bx0 = 0, by0 = 0, bz0 = 0;
-    if (BOX && !last) {  // uniform over the block
-      if (threadIdx.x == 0) {
-        int fi, fj, fk;
-        if (b.blag) {
-          unpack_site(b.blag[first], S.qkb, S.qjb, fi, fj, fk);
-        } else {
-          lattice_ijk(S, first - S.p_off, fi, fj, fk);
-        }
-        const float3 fx = mesh_pos(S, fi, fj, fk, ld3(b.bd, first));
-        box_org[0] = cic_axis(fx.x, S.mx).i0 - 2;
-        box_org[1] = (cic_axis(fx.y, S.my).i0 & ~15) - 2;
-        box_org[2] = (cic_axis(fx.z, S.mz).i0 & ~15) - 4;
-      }
-      for (int q = threadIdx.x; q < BN / 4; q += kThreads)
-        reinterpret_cast<float4*>(box)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-      __syncthreads();
-      bx0 = box_org[0];
-      by0 = box_org[1];
-      bz0 = box_org[2];
-    }
 #pragma unroll 1
     for (int item = 0; item < kItems; ++item) {
       const int64_t i = first + item * kThreads + threadIdx.x;
@@ -659,8 +598,7 @@ k_step_sorted(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
         w[2 * q] = __fmul_rn(c1.wxy[q], c1.wz0);
         w[2 * q + 1] = __fmul_rn(c1.wxy[q], c1.wz1);
       }
-      const unsigned heads =
-          FPM_SORTED_SEGSUM ? __ballot_sync(0xffffffffu, head) : 0xffffffffu;
+      const unsigned heads = __ballot_sync(0xffffffffu, head);
       if (heads != 0xffffffffu) {
         // segmented sums over runs of contiguous lanes with equal keys (a
         // key can recur in a later run after the particles drifted since
@@ -681,71 +619,7 @@ k_step_sorted(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
           }
         }
       }
-      // z-adjacent runs share four cells: the run whose base cell is one z
-      // step past the previous run's takes that run's upper-z weights into
-      // its lower-z ones, and the previous run leaves them out
-      bool skip_z1 = false;
-      if (FPM_SORTED_ZMERGE) {
-        const bool nowrap = valid && c1.z1 == c1.z0 + 1;
-        const int ph = lane > 0 ? run_head(heads, lane - 1) : 0;
-        const unsigned above = heads & ~((2u << lane) - 1u);
-        const int nh = above ? __ffs(above) - 1 : lane;
-        const unsigned kp = __shfl_sync(0xffffffffu, key, ph);
-        const int pnw = __shfl_sync(0xffffffffu, (int)nowrap, ph);
-        const unsigned kn = __shfl_sync(0xffffffffu, key, nh);
-        const int nv = __shfl_sync(0xffffffffu, (int)valid, nh);
-        const bool take = head && valid && lane > 0 && pnw && kp + 1u == key;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float t = __shfl_sync(0xffffffffu, w[2 * q + 1], ph);
-          if (take) w[2 * q] = __fadd_rn(w[2 * q], t);
-        }
-        skip_z1 = nh != lane && nv && nowrap && key + 1u == kn;
-      }
-      if (valid && (head || !FPM_SORTED_SEGSUM)) {
-        if (BOX) {
-          const int rx0 = box_rel(nx1.i0, bx0, S.mx),
-                    rx1 = box_rel(nx1.i1, bx0, S.mx),
-                    ry0 = box_rel(ny1.i0, by0, S.my),
-                    ry1 = box_rel(ny1.i1, by0, S.my),
-                    rz0 = box_rel(nz1.i0, bz0, S.mz),
-                    rz1 = box_rel(nz1.i1, bz0, S.mz);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int rx = (q & 1) ? rx1 : rx0, ry = (q >> 1) ? ry1 : ry0;
-            const bool in = (unsigned)rx < (unsigned)BX &&
-                            (unsigned)ry < (unsigned)BY;
-            float* t = box + (rx * BY + ry) * BZ;
-            if (in && (unsigned)rz0 < (unsigned)BZ)
-              atomicAdd(t + rz0, w[2 * q]);
-            else
-              red_add(m + c1.row[q] + c1.z0, w[2 * q]);
-            if (in && (unsigned)rz1 < (unsigned)BZ)
-              atomicAdd(t + rz1, w[2 * q + 1]);
-            else
-              red_add(m + c1.row[q] + c1.z1, w[2 * q + 1]);
-          }
-        } else {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            red_add(m + c1.row[q] + c1.z0, w[2 * q]);
-            if (!skip_z1) red_add(m + c1.row[q] + c1.z1, w[2 * q + 1]);
-          }
-        }
-      }
-    }
-    if (BOX && !last) {  // flush the box
-      __syncthreads();
-      for (int q = threadIdx.x; q < BN / 4; q += kThreads) {
-        const float4 v = reinterpret_cast<const float4*>(box)[q];
-        if (v.x == 0.f && v.y == 0.f && v.z == 0.f && v.w == 0.f) continue;
-        const int zg = q % (BZ / 4), row = q / (BZ / 4);
-        const int cy = wrap_near(by0 + row % BY, S.my);
-        const int cx = wrap_near(bx0 + row / BY, S.mx);
-        const int cz = wrap_near(bz0 + 4 * zg, S.mz);
-        red_add_f4(m + ((int64_t)cx * S.my + cy) * S.mz + cz, v);
-      }
-      __syncthreads();  // the next chunk zeroes the box
+      if (valid && head) paint_rows(m, S.pairs, c1, w);
     }
   }
 }
@@ -755,13 +629,8 @@ k_step_sorted(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
 void launch_step_sorted(const SimDev* sims, int nsims, int64_t ch0,
                         int64_t ch1, const BinStepArgs& b, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  // the shared-memory box follows tiles of 16 cells
-  if (FPM_SORTED_BOX && b.tile_log2 == 4)
-    launch_pdl(k_step_sorted<true>, dim3(grid_for(ch1 - ch0)), dim3(kThreads),
-               0, st, sims, nsims, ch0, ch1, b);
-  else
-    launch_pdl(k_step_sorted<false>, dim3(grid_for(ch1 - ch0)),
-               dim3(kThreads), 0, st, sims, nsims, ch0, ch1, b);
+  launch_pdl(k_step_sorted, dim3(grid_for(ch1 - ch0)), dim3(kThreads), 0, st,
+             sims, nsims, ch0, ch1, b);
 }
 
 void launch_step_binned(int tile, const SimDev* sims, int nsims, int64_t ch0,

@@ -289,11 +289,16 @@ __device__ __forceinline__ void cols_dft(float2* P) {
 #endif
 constexpr int kPlaneThreads = FPM_PLANE_THREADS;  // threads of the plane kernels
 
-template <int NY, int M>
+//
+// PAIRS: rho holds the painted z pairs (paint_rows, two floats per cell)
+// and the density is formed as the plane is loaded, rho[z] = P[z].x +
+// P[z - 1].y: one float4 is a complex value's two pairs, the y before them
+// comes from the lane below (or, at a warp's or a row's start, a load).
+template <int NY, int M, bool PAIRS>
 __global__ void __launch_bounds__(kPlaneThreads)
 k_fft_plane_fwd(const SimDev* __restrict__ sims, int first, int nx,
                 float* __restrict__ rho, float2* __restrict__ dk,
-                int zero_rho) {
+                int painted, int zero_rho) {
   pdl_wait();  // the density painted before
   extern __shared__ float2 P[];  // NY rows of M + 1
   constexpr int T = kPlaneThreads;
@@ -301,21 +306,38 @@ k_fft_plane_fwd(const SimDev* __restrict__ sims, int first, int nx,
   const int s = first + blockIdx.x / nx;
   const int x = blockIdx.x % nx;
   const SimDev& S = sims[s];
-  float4* src = reinterpret_cast<float4*>(rho + S.m_off + (int64_t)x * NY * 2 * M);
+  constexpr int NF = PAIRS ? 2 : 1;       // floats per cell
+  constexpr int NV = NF * NY * M / 2;     // float4 per plane
+  float* plane = rho + (painted ? S.r_off : S.m_off) +
+                 (int64_t)x * NY * NF * 2 * M;
+  float4* src = reinterpret_cast<float4*>(plane);
   float2* dst = dk + S.s_off + (int64_t)x * NY * NZH;
-  constexpr int NV = NY * M / 2;  // float4 (two complex) per plane
+  if (PAIRS) {
+    static_assert(NV % 32 == 0, "whole warps");
+    const int lane = threadIdx.x & 31;
 #pragma unroll 8
-  for (int e = threadIdx.x; e < NV; e += T) {
-    const float4 v = src[e];
-    const int r = (2 * e) / M, m = (2 * e) % M;
-    P[r * NZH + m] = make_float2(v.x, v.y);
-    P[r * NZH + m + 1] = make_float2(v.z, v.w);
+    for (int e = threadIdx.x; e < NV; e += T) {
+      const float4 v = src[e];
+      const int r = e / M, m = e % M;
+      float y = __shfl_up_sync(0xffffffffu, v.w, 1);
+      if (lane == 0 || m == 0)
+        y = plane[4 * (m ? e - 1 : e + M - 1) + 3];
+      P[r * NZH + m] = make_float2(__fadd_rn(v.x, y), __fadd_rn(v.z, v.y));
+    }
+  } else {
+#pragma unroll 8
+    for (int e = threadIdx.x; e < NV; e += T) {
+      const float4 v = src[e];
+      const int r = (2 * e) / M, m = (2 * e) % M;
+      P[r * NZH + m] = make_float2(v.x, v.y);
+      P[r * NZH + m + 1] = make_float2(v.z, v.w);
+    }
   }
+  __syncthreads();  // the whole plane has been read
   if (zero_rho) {
     for (int e = threadIdx.x; e < NV; e += T)
       src[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  __syncthreads();
   rows_fwd<M, T>(P, NY, NZH);
   // real-to-complex unpacking, one (k, M - k) pair per work item
   constexpr int KP = M / 2 + 1;
@@ -450,9 +472,9 @@ k_fft_columns(const SimDev* __restrict__ sims, int first, int nblk,
 // DFTs (cols_dft), a twiddle W_NX^(a kb) and R-point DFTs in registers,
 // where the transfer function is applied and the inverse starts; the
 // column block moves through shared memory as rows of kXCols modes.  With
-// rho_zero, the block also zeroes its share of that buffer: zmul floats per
-// cell of the sim (1: the density mesh; 4: the interleaved adjoint force
-// mesh).
+// zero, the block also zeroes its share of that buffer: zmul floats per
+// cell of the sim (1: the painted density, from r_off; 4: the interleaved
+// adjoint force mesh).
 // Columns per x-pass block.  Measured on B200 at 2 x 512^3: 8 columns
 // (64-byte rows, 32 KB) 1.19 ms per pass, 16 (128-byte rows, 64 KB) 1.01
 // ms; a persistent variant with cp.async double buffering of 8-column
@@ -465,7 +487,7 @@ constexpr int kXThreads = 512, kXCols = FPM_XPASS_COLS;
 template <int NX>
 __global__ void __launch_bounds__(kXThreads)
 k_fft_xcols(const SimDev* __restrict__ sims, int first, int nblk,
-            const float2* in, float2* out, float* __restrict__ rho_zero,
+            const float2* in, float2* out, float* __restrict__ zero,
             int zmul, AxisTabs tabs, Green G,
             const int32_t* __restrict__ nsteps, int pos) {
   constexpr int R = NX / 64, C = kXCols, T = kXThreads;
@@ -489,10 +511,11 @@ k_fft_xcols(const SimDev* __restrict__ sims, int first, int nblk,
     const int e = threadIdx.x + i * T;
     b4[e] = src[(int64_t)(e / (C / 2)) * rstride + e % (C / 2)];
   }
-  if (rho_zero) {  // this block's share, in float4
+  if (zero) {  // this block's share, in float4
     const int64_t q4 = (int64_t)zmul * S.mx * S.my * S.mz / 4;
     const int64_t per = (q4 + nblk - 1) / nblk;
-    float4* r4 = reinterpret_cast<float4*>(rho_zero + zmul * S.m_off);
+    float4* r4 = reinterpret_cast<float4*>(
+        zero + (zmul == 1 ? S.r_off : zmul * S.m_off));
     const int64_t e1 = min(q4, (blk + 1) * per);
     for (int64_t e = blk * per + threadIdx.x; e < e1; e += T)
       r4[e] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -708,7 +731,10 @@ bool g_tw_ready[64] = {};
 template <int NY, int M>
 int set_plane_smem() {
   const int bytes = NY * (M + 1) * (int)sizeof(float2);
-  if (cudaFuncSetAttribute(k_fft_plane_fwd<NY, M>,
+  if (cudaFuncSetAttribute(k_fft_plane_fwd<NY, M, true>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           bytes) != cudaSuccess ||
+      cudaFuncSetAttribute(k_fft_plane_fwd<NY, M, false>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize,
                            bytes) != cudaSuccess ||
       cudaFuncSetAttribute(k_fft_plane_inv<NY, M, kOutStencil>,
@@ -742,15 +768,18 @@ int prepare_ny(int M) {
   return FPM_ERR_UNSUPPORTED;
 }
 
-// The kernels of one mesh shape (NY, M = nz / 2).
+// The kernels of one mesh shape (NY, M = nz / 2).  rho: the painted density
+// (pairs: z pairs), or with real_out a plain mesh.
 template <int NY, int M>
 void launch_shape(const SimDev* sims, int first, int n, int nx, float* rho,
-                  int zero_rho, float2* dk, float2* fk, float* fmesh,
+                  bool pairs, int zero_rho, float2* dk, float2* fk, float* fmesh,
                   float* phi, AxisTabs tabs, const Green& G, bool grad3,
                   bool real_out, cudaStream_t st) {
   const size_t smem = (size_t)NY * (M + 1) * sizeof(float2);
-  launch_pdl(k_fft_plane_fwd<NY, M>, dim3(n * nx), dim3(kPlaneThreads), smem,
-             st, sims, first, nx, rho, dk, zero_rho);
+  auto fwd = pairs ? k_fft_plane_fwd<NY, M, true>
+                   : k_fft_plane_fwd<NY, M, false>;
+  launch_pdl(fwd, dim3(n * nx), dim3(kPlaneThreads), smem, st, sims, first, nx,
+             rho, dk, real_out ? 0 : 1, zero_rho);
   const int ncols = NY * (M + 1);
   if (!grad3 && nx == 128) {
     // x DFT, potential, inverse x DFT by the x-pass kernel (R = 2): four
@@ -802,14 +831,14 @@ void launch_shape(const SimDev* sims, int first, int n, int nx, float* rho,
 
 template <int NY>
 void launch_ny(int M, const SimDev* sims, int first, int n, int nx,
-               float* rho, int zero_rho, float2* dk, float2* fk, float* fmesh,
-               float* phi, AxisTabs tabs, const Green& G, bool grad3,
+               float* rho, bool pairs, int zero_rho, float2* dk, float2* fk,
+               float* fmesh, float* phi, AxisTabs tabs, const Green& G, bool grad3,
                bool real_out, cudaStream_t st) {
   switch (M) {
 #define FPM_SHAPE_CASE(MM)                                                  \
   case MM:                                                                  \
-    launch_shape<NY, MM>(sims, first, n, nx, rho, zero_rho, dk, fk, fmesh,  \
-                         phi, tabs, G, grad3, real_out, st);                \
+    launch_shape<NY, MM>(sims, first, n, nx, rho, pairs, zero_rho, dk, fk,  \
+                         fmesh, phi, tabs, G, grad3, real_out, st);         \
     break;
     FPM_FFT_HALF(FPM_SHAPE_CASE)
 #undef FPM_SHAPE_CASE
@@ -857,16 +886,16 @@ int fft_fused_prepare(int nx, int ny, int nz) {
 }
 
 void launch_fft_force(const SimDev* sims, int first, int n, int nx, int ny,
-                      int nz, float* rho, int zero_rho, float2* dk,
-                      float2* fk, float* fmesh, float* phi, AxisTabs tabs,
+                      int nz, float* rho, bool pairs, int zero_rho,
+                      float2* dk, float2* fk, float* fmesh, float* phi, AxisTabs tabs,
                       const Green& G, bool grad3, cudaStream_t st) {
   if (n <= 0) return;
   g_launches.fetch_add(grad3 ? 3 : 4, std::memory_order_relaxed);
   switch (ny) {
 #define FPM_NY_CASE(NN)                                                      \
   case NN:                                                                   \
-    launch_ny<NN>(nz / 2, sims, first, n, nx, rho, zero_rho, dk, fk, fmesh,  \
-                  phi, tabs, G, grad3, false, st);                           \
+    launch_ny<NN>(nz / 2, sims, first, n, nx, rho, pairs, zero_rho, dk, fk,  \
+                  fmesh, phi, tabs, G, grad3, false, st);                    \
     break;
     FPM_FFT_SIZES(FPM_NY_CASE)
 #undef FPM_NY_CASE
@@ -883,7 +912,7 @@ void launch_fft_potential(const SimDev* sims, int first, int n, int nx,
   switch (ny) {
 #define FPM_NY_CASE(NN)                                                   \
   case NN:                                                                \
-    launch_ny<NN>(nz / 2, sims, first, n, nx, src, 0, dk, nullptr,        \
+    launch_ny<NN>(nz / 2, sims, first, n, nx, src, false, 0, dk, nullptr, \
                   nullptr, out, tabs, G, false, true, st);                \
     break;
     FPM_FFT_SIZES(FPM_NY_CASE)
@@ -930,7 +959,7 @@ int fft_xpass_prepare() {
 }
 
 void launch_fft_xpass(const SimDev* sims, int first, int n, int nx, int ny,
-                      int nzh, const float2* in, float2* out, float* rho_zero,
+                      int nzh, const float2* in, float2* out, float* zero,
                       int zmul, AxisTabs tabs, const Green& G,
                       const int32_t* nsteps, int pos, cudaStream_t st) {
   if (n <= 0) return;
@@ -939,10 +968,10 @@ void launch_fft_xpass(const SimDev* sims, int first, int n, int nx, int ny,
   const unsigned grid = (unsigned)(n * nblk);
   if (nx == 512)
     k_fft_xcols<512><<<grid, kXThreads, xpass_smem(512), st>>>(
-        sims, first, nblk, in, out, rho_zero, zmul, tabs, G, nsteps, pos);
+        sims, first, nblk, in, out, zero, zmul, tabs, G, nsteps, pos);
   else
     k_fft_xcols<256><<<grid, kXThreads, xpass_smem(256), st>>>(
-        sims, first, nblk, in, out, rho_zero, zmul, tabs, G, nsteps, pos);
+        sims, first, nblk, in, out, zero, zmul, tabs, G, nsteps, pos);
 }
 
 }  // namespace fpm

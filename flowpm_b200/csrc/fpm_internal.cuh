@@ -39,6 +39,8 @@ struct SimDev {
   int64_t np;            // particles
   int64_t p_off;         // first particle
   int64_t m_off;         // first force-mesh cell
+  int64_t r_off;         // first float of the painted density
+  int pairs;             // painted as z pairs (paint_pairs), else per cell
   int64_t s_off;         // first force-mesh half-spectrum mode
   int64_t l_off;         // first lattice cell
   int64_t ls_off;        // first lattice half-spectrum mode
@@ -249,6 +251,13 @@ __device__ __forceinline__ void red_add_f4(float* p, float4 v) {
                : "memory");
 }
 
+// p[0..1] += (a, b) as one 8-byte vector reduction (p 8-byte aligned).
+__device__ __forceinline__ void red_add_f2(float* p, float a, float b) {
+  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(a),
+               "f"(b)
+               : "memory");
+}
+
 // p[0..2] += (a, b, c) as one 16-byte vector reduction (p 16-byte aligned;
 // p[3] += 0).
 __device__ __forceinline__ void red_add_v4(float* p, float a, float b,
@@ -259,9 +268,6 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b,
 }
 
 // Tuning knobs of the particle kernels (compile-time).
-#ifndef FPM_STEP_BLOCKED
-#define FPM_STEP_BLOCKED 1  // the particle kernels walk lattice blocks
-#endif
 // Measured on B200, k_step per leapfrog step at 128^3 / 256^3: 3 blocks
 // (80 registers) 87.4 / 621 us, 4 blocks (64) 84.6 / 594, 5 blocks (48)
 // 85.4 / 583, 6 blocks (40, spills) 96.1 / 657.  The v4 pair reduction is
@@ -457,10 +463,46 @@ __device__ __forceinline__ void paint_cic8(float* __restrict__ m,
   }
 }
 
-__device__ __forceinline__ void paint8(float* __restrict__ m, int mx, int my,
-                                       int mz, const Axis& ax, const Axis& ay,
-                                       const Axis& az) {
-  paint_cic8(m, cic8(ax, ay, az, my, mz), 1.f);
+// Deposit of the step kernels into a simulation's painted density m; w[2 q],
+// w[2 q + 1]: the weights of row q.
+//
+// pairs: two floats per cell, P[c].x the deposits into cell c made as lower z
+// neighbour, P[c].y those made as upper z neighbour by the particles of cell
+// c, which belong to the next cell along z: rho[z] = P[z].x + P[z - 1].y
+// (periodic).  The two z neighbours of each of a particle's four (x, y) rows
+// are then one aligned 8-byte reduction whatever the parity of z: four
+// reductions instead of eight.  The particle kernels are bound by the
+// sectors that the reductions send from L1 to L2 (21 per warp-wide scalar
+// reduction on the lattice walk at 128^3, 59 % of the L1's request cycles):
+// k_step on the walk 88 -> 71 us at 128^3 and 4.70 -> 3.65 ms at 512^3, the
+// pairs' read and clearing in the solve 3 us and 0.3 ms.  Only simulations
+// with one cell per particle (pm_nc_factor 1) paint pairs: a finer mesh has
+// more cells to read back (128^3 particles on 256^3: k_step 118 us per cell,
+// 125 us in pairs, and 48 us more in the solve).
+__device__ __forceinline__ void paint_rows(float* __restrict__ m, int pairs,
+                                           const Cic8& c, const float* w) {
+  if (pairs) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      red_add_f2(m + 2 * (size_t)(c.row[q] + c.z0), w[2 * q], w[2 * q + 1]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      red_add(m + c.row[q] + c.z0, w[2 * q]);
+      red_add(m + c.row[q] + c.z1, w[2 * q + 1]);
+    }
+  }
+}
+
+__device__ __forceinline__ void paint8(float* __restrict__ m, int pairs,
+                                       const Cic8& c) {
+  float w[8];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    w[2 * q] = __fmul_rn(c.wxy[q], c.wz0);
+    w[2 * q + 1] = __fmul_rn(c.wxy[q], c.wz1);
+  }
+  paint_rows(m, pairs, c, w);
 }
 
 // Deposit s * W at the 8 neighbours.
@@ -520,37 +562,29 @@ __device__ __forceinline__ void mode_ijl(int64_t local, int ny, int nzh,
 }
 
 // Chunk kind and particle enumeration of the particle kernels that gather
-// from or scatter to the meshes (lattice blocks when FPM_STEP_BLOCKED, else
-// kChunk consecutive particles).
-constexpr int kTraverse = FPM_STEP_BLOCKED ? kBlock : kPart;
+// from or scatter to the meshes: lattice blocks.
+constexpr int kTraverse = kBlock;
 
 __device__ __forceinline__ int64_t traverse_first(const SimDev& S) {
-  return FPM_STEP_BLOCKED ? S.ch_b : S.ch_p;
+  return S.ch_b;
 }
 
-// One chunk of the traversal: the lattice origin of its block (blocked
-// traversal) or its first flat particle.  Built once per chunk, so the
-// divisions by the block counts are not repeated per particle.
+// One chunk of the traversal: the lattice origin of its block.  Built once
+// per chunk, so the divisions by the block counts are not repeated per
+// particle.
 struct Walk {
   int i0, j0, k0;
-  int64_t base;
 };
 
 // Chunk `rel` (relative to the sim's first chunk).
 __device__ __forceinline__ Walk walk_chunk(const SimDev& S, int64_t rel) {
   Walk w;
-#if FPM_STEP_BLOCKED
   const unsigned b = (unsigned)rel;
   const unsigned r = b / (unsigned)S.nbk;
   const unsigned bi = r / (unsigned)S.nbj;
   w.i0 = (int)bi * kPlanes * S.wi;
   w.j0 = (int)(r - bi * (unsigned)S.nbj) * kBJ;
   w.k0 = (int)(b - r * (unsigned)S.nbk) * kBK;
-  w.base = 0;
-#else
-  w.i0 = w.j0 = w.k0 = 0;
-  w.base = rel * kChunk;
-#endif
   return w;
 }
 
@@ -563,19 +597,12 @@ __device__ __forceinline__ bool walk_particle(const SimDev& S, const Walk& w,
                                               int item, int& i, int& j,
                                               int& k, int64_t& local) {
   const int t = threadIdx.x + item * kThreads;
-#if FPM_STEP_BLOCKED
   i = w.i0 + t / (kBJ * kBK);
   j = w.j0 + (t / kBK) % kBJ;
   k = w.k0 + t % kBK;
   local = (int64_t)(((unsigned)i * (unsigned)S.ny + (unsigned)j) *
                         (unsigned)S.nz + (unsigned)k);
   return i < S.nx && j < S.ny && k < S.nz;
-#else
-  local = w.base + t;
-  if (local >= S.np) return false;
-  lattice_ijk(S, local, i, j, k);
-  return true;
-#endif
 }
 
 inline unsigned grid_for(int64_t chunks) {

@@ -4,6 +4,7 @@
 // elements; a chunk never straddles two simulations, and the owning
 // simulation is found by binary search over the per-sim first chunk, so the
 // same launch advances a batch of simulations of different sizes.
+#include <algorithm>
 #include <atomic>
 
 #include "fpm_kernels.cuh"
@@ -21,7 +22,7 @@ k_paint_lattice(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
   for (int64_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
     const SimDev S = sims[find_sim(sims, nsims, ch, kTraverse)];
     const Walk w = walk_chunk(S, ch - traverse_first(S));
-    float* m = rho + S.m_off;
+    float* m = rho + S.r_off;
 #pragma unroll 4
     for (int it = 0; it < S.wi; ++it) {
       int i, j, k;
@@ -30,8 +31,8 @@ k_paint_lattice(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
       const float3 d = ld3(disp, S.p_off + local);
       const float3 x = mesh_pos(S, i, j, k, d);
       if (!finite3(x.x, x.y, x.z)) atomicOr(status, FPM_STATUS_NONFINITE_POS);
-      paint8(m, S.mx, S.my, S.mz, cic_axis(x.x, S.mx), cic_axis(x.y, S.my),
-             cic_axis(x.z, S.mz));
+      paint8(m, S.pairs, cic8(cic_axis(x.x, S.mx), cic_axis(x.y, S.my),
+                              cic_axis(x.z, S.mz), S.my, S.mz));
     }
   }
 }
@@ -53,7 +54,7 @@ k_step(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
     const float fac = a.ffac[s];
     const float invb = 1.0f / (float)S.bf;
     const int64_t mcells = (int64_t)S.mx * S.my * S.mz;
-    float* m = a.rho + S.m_off;
+    float* m = a.rho + S.r_off;
     const Walk w = walk_chunk(S, ch - traverse_first(S));
 #pragma unroll 1
     for (int it = 0; it < S.wi; ++it) {
@@ -102,16 +103,16 @@ k_step(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
       }
       p = axpy(p, ks, f);  // opening kick of step it
       d = axpy(d, dr, p);  // drift of step it
-      const float3 xn = mesh_pos(S, i, j, k, d);
       if (valid) {
         st3(a.mom, g, p);
         st3(a.disp, g, d);
-        if (!finite3(xn.x, xn.y, xn.z))
-          atomicOr(a.status, FPM_STATUS_NONFINITE_POS);
       }
+      const float3 xn = mesh_pos(S, i, j, k, d);
+      if (valid && !finite3(xn.x, xn.y, xn.z))
+        atomicOr(a.status, FPM_STATUS_NONFINITE_POS);
       const Cic8 c1 = cic8(cic_axis(xn.x, S.mx), cic_axis(xn.y, S.my),
                            cic_axis(xn.z, S.mz), S.my, S.mz);
-      if (valid) paint_cic8(m, c1, 1.f);
+      if (valid) paint8(m, S.pairs, c1);
     }
   }
 }
@@ -136,7 +137,7 @@ k_pgd(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
         pgd[((int64_t)s * pgd_stride + (nsteps ? pos : 0)) * 3];
     const float b = (float)S.bf;
     const int64_t mcells = (int64_t)S.mx * S.my * S.mz;
-    float* m = rho + S.m_off;
+    float* m = rho + S.r_off;
     const Walk w = walk_chunk(S, ch - traverse_first(S));
 #pragma unroll 1
     for (int it = 0; it < S.wi; ++it) {
@@ -156,8 +157,8 @@ k_pgd(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
       st3(disp, g, d);
       const float3 xn = mesh_pos(S, i, j, k, d);
       if (!finite3(xn.x, xn.y, xn.z)) atomicOr(status, FPM_STATUS_NONFINITE_POS);
-      paint8(m, S.mx, S.my, S.mz, cic_axis(xn.x, S.mx), cic_axis(xn.y, S.my),
-             cic_axis(xn.z, S.mz));
+      paint8(m, S.pairs, cic8(cic_axis(xn.x, S.mx), cic_axis(xn.y, S.my),
+                              cic_axis(xn.z, S.mz), S.my, S.mz));
     }
   }
 }
@@ -196,6 +197,72 @@ k_force_readout(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
 // Fourier kernels
 // ---------------------------------------------------------------------------
 
+// The painted z pairs (paint_rows) of the sims [first, first + gridDim.y)
+// of one mesh shape as the plain density that the library transforms read,
+// rho[z] = P[z].x + P[z - 1].y; with zero, the pairs are cleared on the way
+// for the next paint.  One warp per row along z, NC cells per lane (2 when
+// mz and r_off / 2 are even, else 1), kRowPasses passes of the row loaded
+// before any is used; the row's last pair is read first, so that a row is
+// cleared only by the warp that has read it.
+constexpr int kRowPasses = 4;
+
+template <int NC>
+__global__ void __launch_bounds__(kThreads)
+k_pair_density(const SimDev* __restrict__ sims, int first, int nrows, int mz,
+               float* __restrict__ pairs, float* __restrict__ rho, int zero,
+               const int32_t* __restrict__ nsteps, int pos) {
+  const int s = first + blockIdx.y;
+  if (nsteps && pos > nsteps[s]) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t m_off = sims[s].m_off, r_off = sims[s].r_off;
+  for (int r = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); r < nrows;
+       r += gridDim.x * (kThreads / 32)) {
+    float* P = pairs + r_off + (int64_t)r * 2 * mz;
+    float* o = rho + m_off + (int64_t)r * mz;
+    float prev = P[2 * mz - 1];  // y of the cell before the pass
+    for (int z0 = 0; z0 < mz; z0 += 32 * NC * kRowPasses) {
+      float2 v[kRowPasses][NC];
+#pragma unroll
+      for (int q = 0; q < kRowPasses; ++q) {
+        const int z = z0 + (q * 32 + lane) * NC;
+        if (z < mz) {
+          if (NC == 2) {
+            const float4 a = *reinterpret_cast<const float4*>(P + 2 * z);
+            v[q][0] = make_float2(a.x, a.y);
+            v[q][NC - 1] = make_float2(a.z, a.w);
+          } else {
+            v[q][0] = *reinterpret_cast<const float2*>(P + 2 * z);
+          }
+        } else {
+          v[q][0] = v[q][NC - 1] = make_float2(0.f, 0.f);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kRowPasses; ++q) {
+        const int z = z0 + (q * 32 + lane) * NC;
+        const float last = v[q][NC - 1].y;
+        float y = __shfl_up_sync(0xffffffffu, last, 1);
+        if (lane == 0) y = prev;
+        prev = __shfl_sync(0xffffffffu, last, 31);
+        if (z < mz) {
+          const float a = __fadd_rn(v[q][0].x, y);
+          if (NC == 2) {
+            *reinterpret_cast<float2*>(o + z) =
+                make_float2(a, __fadd_rn(v[q][NC - 1].x, v[q][0].y));
+            if (zero)
+              *reinterpret_cast<float4*>(P + 2 * z) =
+                  make_float4(0.f, 0.f, 0.f, 0.f);
+          } else {
+            o[z] = a;
+            if (zero)
+              *reinterpret_cast<float2*>(P + 2 * z) = make_float2(0.f, 0.f);
+          }
+        }
+      }
+    }
+  }
+}
+
 // Force spectra, flowpm/tfpm.py:199-215 apply_longrange:
 //   pot_k = delta_k * lap * longrange;  force_d = pot_k * (i g_d)
 // with delta_k = R2C(rho) / (nbar N^3), lap = 1/k^2 rounded to float (0 at
@@ -203,8 +270,7 @@ k_force_readout(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
 __global__ void __launch_bounds__(kThreads)
 k_fourier_force(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
                 const float2* __restrict__ dk, float2* __restrict__ fk,
-                float* __restrict__ rho_zero, AxisTabs tabs, double r2,
-                int deconv, const int32_t* __restrict__ nsteps, int pos,
+                AxisTabs tabs, double r2, int deconv, const int32_t* __restrict__ nsteps, int pos,
                 int skip_fused) {
   for (int64_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
     const int s = find_sim(sims, nsims, ch, kSpec);
@@ -249,11 +315,6 @@ k_fourier_force(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
         o1[local] = make_float2(-__fmul_rn(pi, g1), __fmul_rn(pr, g1));
         o2[local] = make_float2(-__fmul_rn(pi, g2), __fmul_rn(pr, g2));
       }
-      // Zero the density mesh for the next paint (2 cells per mode slot).
-      if (rho_zero) {
-        for (int64_t c = local; c < mcells; c += nmodes)
-          rho_zero[S.m_off + c] = 0.f;
-      }
     }
   }
 }
@@ -264,12 +325,10 @@ k_fourier_force(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
 // gradient i (8 sin k - sin 2k) / 6 of flowpm/kernels.py:72-76 is applied
 // afterwards in real space, where it is exactly the stencil
 // (8 (phi[x+1] - phi[x-1]) - (phi[x+2] - phi[x-2])) / 12 (k_stencil_grad).
-// Also zeroes rho for the next paint.  Used unchanged (rho_zero = null) for
-// the adjoint, the transfer function being real.
+// Used unchanged for the adjoint, the transfer function being real.
 __global__ void __launch_bounds__(kThreads)
 k_fourier_potential(const SimDev* __restrict__ sims, int nsims,
                     int64_t nchunks, const float2* dk, float2* out,
-                    float* __restrict__ rho_zero,
                     AxisTabs tabs, Green G,
                     const int32_t* __restrict__ nsteps, int pos,
                     int skip_fused) {
@@ -302,10 +361,6 @@ k_fourier_potential(const SimDev* __restrict__ sims, int nsims,
         dv.x = __fmul_rn(dv.x, pre);
         dv.y = __fmul_rn(dv.y, pre);
         o[local] = make_float2(__fmul_rn(dv.x, w), __fmul_rn(dv.y, w));
-      }
-      if (rho_zero) {
-        for (int64_t c = local; c < mcells; c += nmodes)
-          rho_zero[S.m_off + c] = 0.f;
       }
     }
   }
@@ -971,26 +1026,37 @@ void launch_paint_lattice(const SimDev* sims, int nsims, int64_t nchunks,
                                                           disp, rho, status);
 }
 
+void launch_pair_density(const SimDev* sims, int first, int n, int mx, int my,
+                         int mz, bool even, float* pairs, float* rho, int zero,
+                         const int32_t* nsteps, int pos, cudaStream_t st) {
+  if (n <= 0) return;
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  const int nrows = mx * my;
+  const dim3 grid(std::min((nrows + 7) / 8, kNumSMs * 16), (unsigned)n);
+  auto k = even ? k_pair_density<2> : k_pair_density<1>;
+  k<<<grid, kThreads, 0, st>>>(sims, first, nrows, mz, pairs, rho, zero,
+                               nsteps, pos);
+}
+
 void launch_fourier_force(const SimDev* sims, int nsims, int64_t nchunks,
-                          const float2* dk, float2* fk, float* rho_zero,
+                          const float2* dk, float2* fk,
                           AxisTabs tabs, double r_split2, int deconv,
                           const int32_t* nsteps, int pos, int skip_fused,
                           cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   k_fourier_force<<<grid_for(nchunks), kThreads, 0, st>>>(
-      sims, nsims, nchunks, dk, fk, rho_zero, tabs, r_split2, deconv, nsteps,
-      pos, skip_fused);
+      sims, nsims, nchunks, dk, fk, tabs, r_split2, deconv, nsteps, pos,
+      skip_fused);
 }
 
 void launch_fourier_potential(const SimDev* sims, int nsims, int64_t nchunks,
-                              const float2* dk, float2* out, float* rho_zero,
+                              const float2* dk, float2* out,
                               AxisTabs tabs, const Green& G,
                               const int32_t* nsteps, int pos, int skip_fused,
                               cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   k_fourier_potential<<<grid_for(nchunks), kThreads, 0, st>>>(
-      sims, nsims, nchunks, dk, out, rho_zero, tabs, G, nsteps, pos,
-      skip_fused);
+      sims, nsims, nchunks, dk, out, tabs, G, nsteps, pos, skip_fused);
 }
 
 void launch_stencil_grad(const SimDev* sims, int nsims, int64_t nchunks,

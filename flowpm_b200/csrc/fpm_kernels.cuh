@@ -30,27 +30,31 @@ struct StepArgs {
   int it;                  // global iteration 0..max_steps
 };
 
-// Paint every particle at (q + disp) * bf into rho (which must be zeroed).
+// Paint every particle at (q + disp) * bf into the painted density rho
+// (zeroed; sim s from r_off, see paint_rows).
 void launch_paint_lattice(const SimDev* sims, int nsims, int64_t nchunks,
                           const float* disp, float* rho, int32_t* status,
                           cudaStream_t st);
 
+// Plain density of the painted z pairs of the sims [first, first + n) of one
+// mesh shape (even: mz and every r_off / 2 even); zero: clears the pairs.  With
+// nsteps, the sims with nsteps < pos are skipped.
+void launch_pair_density(const SimDev* sims, int first, int n, int mx, int my,
+                         int mz, bool even, float* pairs, float* rho, int zero,
+                         const int32_t* nsteps, int pos, cudaStream_t st);
+
 // R2C output -> three force spectra (Green's function * gradient, optional
-// CIC deconvolution and Gaussian long-range window); also zeroes rho.  With
-// nsteps, simulations with nsteps[s] < pos (finished) are skipped, and with
+// CIC deconvolution and Gaussian long-range window).  With nsteps, simulations with nsteps[s] < pos (finished) are skipped, and with
 // skip_fused those whose force meshes come from the fused solve.
 void launch_fourier_force(const SimDev* sims, int nsims, int64_t nchunks,
-                          const float2* dk, float2* fk, float* rho_zero,
-                          AxisTabs tabs, double r_split2, int deconv,
+                          const float2* dk, float2* fk, AxisTabs tabs, double r_split2, int deconv,
                           const int32_t* nsteps, int pos, int skip_fused,
                           cudaStream_t st);
 
 // Potential spectrum delta_k * pre * w(k) with w the transfer function G
-// (one output per sim, layout of dk); also zeroes rho_zero when given.  The
-// adjoint reuses it as is; the PGD correction passes its own G.
+// (one output per sim, layout of dk).  The adjoint reuses it as is; the PGD correction passes its own G.
 void launch_fourier_potential(const SimDev* sims, int nsims, int64_t nchunks,
-                              const float2* dk, float2* out, float* rho_zero,
-                              AxisTabs tabs, const Green& G,
+                              const float2* dk, float2* out, AxisTabs tabs, const Green& G,
                               const int32_t* nsteps, int pos, int skip_fused,
                               cudaStream_t st);
 
@@ -83,7 +87,8 @@ void launch_stencil_div_tiled(const SimDev* sims, int first, int count,
 // Fused Fourier solve (fpm_fft.cu) for meshes with every axis a power of
 // two in [16, 128]: density -> three force meshes (the transfer function of
 // launch_fourier_force) in three kernels over the sims [first, first + n)
-// of one run (equal shapes); also zeroes rho when zero_rho.  dk and fk are
+// of one run (equal shapes); rho is the painted density (pairs: z pairs, two
+// floats per cell) and is zeroed when zero_rho.  dk and fk are
 // the spectrum scratch (R2C layout, fk three spectra per sim).
 bool fft_fused_supported(int nx, int ny, int nz);
 // Once per shape and device before the first launch (twiddle table, shared
@@ -94,8 +99,8 @@ int fft_fused_prepare(int nx, int ny, int nz);
 // scratch); with grad3 (order-0 gradient) it transforms three force spectra
 // (fk scratch).
 void launch_fft_force(const SimDev* sims, int first, int n, int nx, int ny,
-                      int nz, float* rho, int zero_rho, float2* dk,
-                      float2* fk, float* fmesh, float* phi, AxisTabs tabs,
+                      int nz, float* rho, bool pairs, int zero_rho,
+                      float2* dk, float2* fk, float* fmesh, float* phi, AxisTabs tabs,
                       const Green& G, bool grad3, cudaStream_t st);
 // out = C2R(pre * w(k) * R2C(in)) for the sims [first, first + n) of one
 // run (the adjoint's density cotangent from the potential cotangent); in is
@@ -107,14 +112,14 @@ void launch_fft_potential(const SimDev* sims, int first, int n, int nx,
 // Meshes of 256 or 512 cells along x on the cuFFT path: the x pass between
 // batched (y, z) plane transforms, potential spectrum out = x-pass(in) of
 // the sims [first, first + n) of one run (in == out allowed; with nsteps,
-// the sims with nsteps < pos skip); with rho_zero it also zeroes their
-// part of that buffer, zmul floats per cell (1: density mesh, 4: the
+// the sims with nsteps < pos skip); with zero it also zeroes their part of
+// that buffer, zmul floats per cell (1: the painted density, 4: the
 // interleaved adjoint force mesh).  fft_xpass_prepare uploads its twiddles (once per
 // device).
 bool fft_xpass_supported(int nx, int ny, int nz);
 int fft_xpass_prepare();
 void launch_fft_xpass(const SimDev* sims, int first, int n, int nx, int ny,
-                      int nzh, const float2* in, float2* out, float* rho_zero,
+                      int nzh, const float2* in, float2* out, float* zero,
                       int zmul, AxisTabs tabs, const Green& G,
                       const int32_t* nsteps, int pos, cudaStream_t st);
 

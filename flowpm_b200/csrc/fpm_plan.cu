@@ -79,14 +79,14 @@ struct fpm_plan {
   std::vector<SimDev> sims;
   std::vector<Run> runs;
   SimDev* d_sims = nullptr;
-  int64_t total_np = 0, total_m = 0, total_s = 0, total_l = 0, total_ls = 0;
+  int64_t total_np = 0, total_m = 0, total_r = 0, total_s = 0, total_l = 0, total_ls = 0;
   int64_t ch_p = 0, ch_s = 0, ch_m = 0, ch_l = 0, ch_ls = 0, ch_b = 0;
   // tables
   double* d_kk = nullptr;
   float* d_grad = nullptr;
   float* d_win = nullptr;
   // force-mesh buffers
-  float* rho = nullptr;
+  float* rho = nullptr;     // painted density (SimDev::r_off)
   float2* dk = nullptr;
   float2* fk = nullptr;
   float* fmesh = nullptr;
@@ -184,7 +184,7 @@ Green pgd_green(const fpm_plan* p, int pos, bool single) {
 
 // Chunks of the mesh-touching particle kernels (see kTraverse).
 int64_t traverse_chunks(const fpm_plan* p) {
-  return FPM_STEP_BLOCKED ? p->ch_b : p->ch_p;
+  return p->ch_b;
 }
 
 // Record the next timing event of `kind` on st (no-op unless profiling).
@@ -357,10 +357,12 @@ bool stencil_path(const fpm_plan* p) {
 // The potential spectrum out = pre w(k) in of the sims on the cuFFT path
 // (k_fourier_potential), or, for runs on the x-pass path, the x pass that
 // wraps it (both skip the sims with nsteps < pos when act is given); with
-// rho_zero, their density meshes are zeroed.
-void potential_modes(fpm_plan* p, const float2* in, float2* out,
-                     float* rho_zero, const Green& G, const int32_t* act,
-                     int pos, cudaStream_t st, int zmul = 1) {
+// zero, the x-pass runs also zero their part of that buffer, zmul floats per
+// cell (4: the adjoint force mesh; 1: the painted density, of the runs
+// whose density is not in z pairs).
+void potential_modes(fpm_plan* p, const float2* in, float2* out, float* zero,
+                     int zmul, const Green& G, const int32_t* act, int pos,
+                     cudaStream_t st) {
   bool other = false;
   for (auto& r : p->runs) {
     if (r.fused) continue;
@@ -371,11 +373,35 @@ void potential_modes(fpm_plan* p, const float2* in, float2* out,
     const int n = run_active(r, pos);
     const SimDev& S = p->sims[r.first];
     launch_fft_xpass(p->d_sims, r.first, n, S.mx, S.my, S.mzh, in, out,
-                     rho_zero, zmul, tabs_of(p), G, act, pos, st);
+                     zmul == 1 && S.pairs ? nullptr : zero, zmul, tabs_of(p),
+                     G, act, pos, st);
   }
   if (other)
-    launch_fourier_potential(p->d_sims, p->nsims, p->ch_s, in, out, rho_zero,
+    launch_fourier_potential(p->d_sims, p->nsims, p->ch_s, in, out,
                              tabs_of(p), G, act, pos, 1, st);
+}
+
+// R2C of the painted density of run r's first n sims into dk (library
+// transforms): z pairs become the plain density in the plan's phi buffer
+// first, which the transform may use as scratch; with zero, the painted
+// density is cleared for the next paint.
+int density_modes(fpm_plan* p, const Run& r, int n, int zero,
+                  const int32_t* act, int pos, cudaStream_t st) {
+  const SimDev& S = p->sims[r.first];
+  const cufftHandle h = pick(r, n, r.r2c, r.r2c_n);
+  if (S.pairs) {
+    launch_pair_density(p->d_sims, r.first, n, S.mx, S.my, S.mz,
+                        S.mz % 2 == 0 && S.r_off % 4 == 0, p->rho, p->phi,
+                        zero, act, pos, st);
+    FPM_TRY(launch_ok());
+    return exec_r2c(h, p->phi + S.m_off, p->dk + S.s_off, st);
+  }
+  FPM_TRY(exec_r2c(h, p->rho + S.r_off, p->dk + S.s_off, st));
+  if (zero && !r.xpass)  // else the x pass clears it
+    FPM_CUDA(cudaMemsetAsync(p->rho + S.r_off, 0,
+                             sizeof(float) * (size_t)n * S.mx * S.my * S.mz,
+                             st));
+  return FPM_OK;
 }
 
 // The three force meshes D_d phi of the sims (with act, those with nsteps
@@ -436,7 +462,7 @@ int force_meshes(fpm_plan* p, cudaStream_t st, bool zero_rho, int it = -1,
           FPM_CUDA(cudaStreamWaitEvent(rs, p->ev_fork, 0));
       }
     }
-    launch_fft_force(p->d_sims, r.first, n, S.mx, S.my, S.mz, p->rho,
+    launch_fft_force(p->d_sims, r.first, n, S.mx, S.my, S.mz, p->rho, S.pairs,
                      zero_rho ? 1 : 0, p->dk, p->fk, p->fmesh, phi,
                      tabs_of(p), G, !stencil_path(p), rs);
     ++forked;
@@ -452,20 +478,17 @@ int force_meshes(fpm_plan* p, cudaStream_t st, bool zero_rho, int it = -1,
   }
   for (auto& r : p->runs) {
     if (r.fused) continue;
-    const SimDev& S = p->sims[r.first];
     const int n = run_active(r, it);
     if (n == 0) continue;
-    FPM_TRY(exec_r2c(pick(r, n, r.r2c, r.r2c_n), p->rho + S.m_off,
-                     p->dk + S.s_off, st));
+    FPM_TRY(density_modes(p, r, n, zero_rho ? 1 : 0, act, it, st));
   }
   prof_mark(p, 3, st);
   if (stencil_path(p)) {
-    potential_modes(p, p->dk, p->fk, zero_rho ? p->rho : nullptr, G, act, it,
-                    st);
+    potential_modes(p, p->dk, p->fk, zero_rho ? p->rho : nullptr, 1, G, act,
+                    it, st);
   } else {
     launch_fourier_force(p->d_sims, p->nsims, p->ch_s, p->dk, p->fk,
-                         zero_rho ? p->rho : nullptr, tabs_of(p), r2, deconv,
-                         act, it, 1, st);
+                         tabs_of(p), r2, deconv, act, it, 1, st);
   }
   prof_mark(p, 3, st);
   FPM_TRY(launch_ok());
@@ -512,20 +535,18 @@ int pgd_meshes(fpm_plan* p, cudaStream_t st, int pos, float* phi = nullptr) {
     const SimDev& S = p->sims[r.first];
     const int n = run_active(r, apos);
     if (n == 0) continue;
-    launch_fft_force(p->d_sims, r.first, n, S.mx, S.my, S.mz, p->rho, 1,
-                     p->dk, p->fk, p->fmesh, phi, tabs_of(p), G, false, st);
+    launch_fft_force(p->d_sims, r.first, n, S.mx, S.my, S.mz, p->rho,
+                     S.pairs, 1, p->dk, p->fk, p->fmesh, phi, tabs_of(p), G, false, st);
   }
   FPM_TRY(launch_ok());
   if (!any_cufft) return FPM_OK;
   for (auto& r : p->runs) {
     if (r.fused) continue;
-    const SimDev& S = p->sims[r.first];
     const int n = run_active(r, apos);
     if (n == 0) continue;
-    FPM_TRY(exec_r2c(pick(r, n, r.r2c, r.r2c_n), p->rho + S.m_off,
-                     p->dk + S.s_off, st));
+    FPM_TRY(density_modes(p, r, n, 1, act, apos, st));
   }
-  potential_modes(p, p->dk, p->fk, p->rho, G, act, apos, st);
+  potential_modes(p, p->dk, p->fk, p->rho, 1, G, act, apos, st);
   FPM_TRY(launch_ok());
   for (auto& r : p->runs) {
     if (r.fused) continue;
@@ -618,6 +639,11 @@ int update_schedule(fpm_plan* p, int max_steps, const int32_t* nsteps,
   return FPM_OK;
 }
 
+// Whether two simulations (nx, ny, nz, bf) share a run.
+bool same_dims(const int32_t* a, const int32_t* b) {
+  return a[0] == b[0] && a[1] == b[1] && a[2] == b[2] && a[3] == b[3];
+}
+
 int upload_ffac(fpm_plan* p, const double* force_fac, cudaStream_t st) {
   std::vector<float> f(p->nsims);
   for (int s = 0; s < p->nsims; ++s) f[s] = (float)force_fac[s];
@@ -687,6 +713,13 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
     S.np = (int64_t)S.nx * S.ny * S.nz;
     S.p_off = p->total_np;
     S.m_off = p->total_m;
+    // pairs: one cell per particle; a run starts on 16 bytes (the pairs'
+    // 8-byte reductions, the solve's float4), its simulations contiguous
+    // for the batched transforms
+    S.pairs = S.bf == 1 ? 1 : 0;
+    if (s == 0 || !same_dims(dims + 4 * s, dims + 4 * s - 4))
+      p->total_r = (p->total_r + 3) / 4 * 4;
+    S.r_off = p->total_r;
     S.s_off = p->total_s;
     S.l_off = p->total_l;
     S.ls_off = p->total_ls;
@@ -704,8 +737,7 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
     // position 18.1 / 17.5 / 17.3 / 17.1 ms at wi = 4 / 8 / 16 / 32; at
     // 128^3 wi = 4 is best (k_step 85 / 87 / 97 us at 4 / 8 / 16), larger
     // blocks leaving too few of them for the SMs
-    S.wi = !FPM_STEP_BLOCKED ? kItems
-           : (flags & FPM_PLAN_SMALL_BLOCKS) ? 4
+    S.wi = (flags & FPM_PLAN_SMALL_BLOCKS) ? 4
            : S.np >= ((int64_t)1 << 26) ? FPM_WALK_LARGE
            : S.np >= ((int64_t)1 << 23) ? 8 : 4;
     S.nbi = (S.nx + kPlanes * S.wi - 1) / (kPlanes * S.wi);
@@ -720,6 +752,7 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
     p->ch_ls += (nls + kChunk - 1) / kChunk;
     p->total_np += S.np;
     p->total_m += nm;
+    p->total_r += (S.pairs ? 2 : 1) * nm;
     p->total_s += ns;
     p->total_l += S.np;
     p->total_ls += nls;
@@ -732,10 +765,7 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
     axis_tables(S.ny, order0, kk, grad, win);
     axis_tables(S.nz, order0, kk, grad, win);
     p->sims.push_back(S);
-    if (s > 0 && dims[4 * s] == dims[4 * s - 4] &&
-        dims[4 * s + 1] == dims[4 * s - 3] &&
-        dims[4 * s + 2] == dims[4 * s - 2] &&
-        dims[4 * s + 3] == dims[4 * s - 1]) {
+    if (s > 0 && same_dims(dims + 4 * s, dims + 4 * s - 4)) {
       p->runs.back().count++;
     } else {
       Run r;
@@ -765,7 +795,8 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
     // the fused kernels move density and force planes as float4
     bool aligned = true;
     for (int s = r.first; s < r.first + r.count; ++s)
-      if (p->sims[s].m_off % 4 != 0) aligned = false;
+      if (p->sims[s].m_off % 4 != 0 || p->sims[s].r_off % 4 != 0)
+        aligned = false;
     if (!(flags & FPM_PLAN_CUFFT) && aligned &&
         fft_fused_supported(S0.mx, S0.my, S0.mz) &&
         fft_fused_prepare(S0.mx, S0.my, S0.mz) == FPM_OK) {
@@ -858,7 +889,7 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
   p->d_kk = dalloc<double>(kk.size(), tot, ok);
   p->d_grad = dalloc<float>(grad.size(), tot, ok);
   p->d_win = dalloc<float>(win.size(), tot, ok);
-  p->rho = dalloc<float>(p->total_m, tot, ok);
+  p->rho = dalloc<float>(p->total_r, tot, ok);
   p->dk = dalloc<float2>(p->total_s, tot, ok);
   p->fk = dalloc<float2>(3 * p->total_s, tot, ok);
   p->fmesh = dalloc<float>(3 * p->total_m, tot, ok);
@@ -948,7 +979,7 @@ extern "C" int fpm_force(fpm_plan* p, const float* disp,
   if (!p || !disp || !force_fac || !force) return FPM_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   FPM_TRY(upload_ffac(p, force_fac, st));
-  FPM_CUDA(cudaMemsetAsync(p->rho, 0, sizeof(float) * p->total_m, st));
+  FPM_CUDA(cudaMemsetAsync(p->rho, 0, sizeof(float) * p->total_r, st));
   launch_paint_lattice(p->d_sims, p->nsims, traverse_chunks(p), disp, p->rho,
                        p->d_status, st);
   FPM_TRY(launch_ok());
@@ -1023,7 +1054,7 @@ bool chains_ok(const fpm_plan* p) {
 int64_t run_chunk(const fpm_plan* p, size_t k) {
   if (k >= p->runs.size()) return traverse_chunks(p);
   const SimDev& S = p->sims[p->runs[k].first];
-  return FPM_STEP_BLOCKED ? S.ch_b : S.ch_p;
+  return S.ch_b;
 }
 
 int nbody_chains(fpm_plan* p, StepArgs a, cudaStream_t st) {
@@ -1038,7 +1069,7 @@ int nbody_chains(fpm_plan* p, StepArgs a, cudaStream_t st) {
     for (int it = 0; it <= p->max_steps; ++it) {
       const int n = run_active(r, it);
       if (n == 0) continue;  // every simulation of the run has finished
-      launch_fft_force(p->d_sims, r.first, n, S.mx, S.my, S.mz, p->rho,
+      launch_fft_force(p->d_sims, r.first, n, S.mx, S.my, S.mz, p->rho, S.pairs,
                        it < p->max_steps ? 1 : 0, p->dk, p->fk, p->fmesh,
                        p->tape ? tape_phi(p, it) : p->phi, tabs_of(p), G,
                        !stencil_path(p), rs);
@@ -1176,7 +1207,7 @@ int nbody_flow(fpm_plan* p, StepArgs a, cudaStream_t st) {
       int cur = -1;
       for (int it = 0; it <= r.min_steps; ++it) {
         launch_fft_force(p->d_sims, r.first, r.count, S.mx, S.my, S.mz,
-                         p->rho, it < p->max_steps ? 1 : 0, p->dk, p->fk,
+                         p->rho, S.pairs, it < p->max_steps ? 1 : 0, p->dk, p->fk,
                          p->fmesh, p->tape ? tape_phi(p, it) : p->phi,
                          tabs_of(p), G, !stencil_path(p), rs);
         launch_step_sorted(p->d_sims, p->nsims, run_part_chunk(p, k),
@@ -1241,7 +1272,7 @@ int nbody_binned(fpm_plan* p, StepArgs a, cudaStream_t st) {
       for (int it = 0; it <= p->max_steps; ++it) {
         const int n = run_active(r, it);
         if (n == 0) continue;  // every simulation of the run has finished
-        launch_fft_force(p->d_sims, r.first, n, S.mx, S.my, S.mz, p->rho,
+        launch_fft_force(p->d_sims, r.first, n, S.mx, S.my, S.mz, p->rho, S.pairs,
                          it < p->max_steps ? 1 : 0, p->dk, p->fk, p->fmesh,
                          p->tape ? tape_phi(p, it) : p->phi, tabs_of(p), G,
                          !stencil_path(p), rs);
@@ -1321,7 +1352,7 @@ extern "C" int fpm_nbody_run(fpm_plan* p, float* disp, float* mom,
   a.ckpt_every = ckpt ? ckpt_every : 1;
   a.total_np = p->total_np;
   a.max_steps = p->max_steps;
-  FPM_CUDA(cudaMemsetAsync(p->rho, 0, sizeof(float) * p->total_m, st));
+  FPM_CUDA(cudaMemsetAsync(p->rho, 0, sizeof(float) * p->total_r, st));
   prof_mark(p, 2, st);
   launch_paint_lattice(p->d_sims, p->nsims, traverse_chunks(p), disp, p->rho,
                        p->d_status, st);
@@ -1576,7 +1607,7 @@ extern "C" int fpm_pgd(fpm_plan* p, float* disp, const double* params,
   for (size_t i = 0; i < h.size(); ++i) h[i] = (float)params[i];
   FPM_CUDA(cudaMemcpyAsync(p->d_pgd1, h.data(), sizeof(float) * h.size(),
                            cudaMemcpyHostToDevice, st));
-  FPM_CUDA(cudaMemsetAsync(p->rho, 0, sizeof(float) * p->total_m, st));
+  FPM_CUDA(cudaMemsetAsync(p->rho, 0, sizeof(float) * p->total_r, st));
   launch_paint_lattice(p->d_sims, p->nsims, traverse_chunks(p), disp, p->rho,
                        p->d_status, st);
   FPM_TRY(launch_ok());
@@ -1637,8 +1668,8 @@ static int adjoint_density(fpm_plan* p, int pos, const Green& G,
   if (any_cufft) {
     // on the x-pass path the x pass also clears the adjoint force mesh,
     // which the divergence above has consumed, for the next scatter
-    potential_modes(p, p->dk, p->dk, p->all_xpass ? p->lmesh : nullptr, G,
-                    act, pos, st, 4);
+    potential_modes(p, p->dk, p->dk, p->all_xpass ? p->lmesh : nullptr, 4, G,
+                    act, pos, st);
     FPM_TRY(launch_ok());
     for (auto& r : p->runs) {
       const SimDev& S = p->sims[r.first];
@@ -1690,7 +1721,7 @@ static int adjoint_step(fpm_plan* p, AdjArgs& a, int it, cudaStream_t st) {
     prof_mark(p, 6, st);
     FPM_TRY(launch_ok());
   } else {
-    FPM_CUDA(cudaMemsetAsync(p->rho, 0, sizeof(float) * p->total_m, st));
+    FPM_CUDA(cudaMemsetAsync(p->rho, 0, sizeof(float) * p->total_r, st));
     prof_mark(p, 5, st);
     launch_adj_drift_paint(p->d_sims, p->nsims, traverse_chunks(p), a, st);
     prof_mark(p, 5, st);
