@@ -263,7 +263,10 @@ def _potential_tape(dims, T, store, device, pgd=False):
   plan's force-mesh cells (with PGD, also T PGD potentials and T particle
   displacements; the layout of fpm_nbody_set_tape), or None.  store: True,
   False, or None for automatic (when it takes under a quarter of the free
-  device memory)."""
+  device memory).  Asking the driver for the free memory takes 1.3 ms, as
+  long as the gradient of a small simulation, so a tape under 1/1024 of the
+  device's memory (187 MB on a B200) is allocated without asking, and left
+  out if that fails."""
   if store is False:
     return None
   cells = sum((b * nx) * (b * ny) * (b * nz) for nx, ny, nz, b in dims)
@@ -274,6 +277,12 @@ def _potential_tape(dims, T, store, device, pgd=False):
   if store is None:
     if cells % 4:  # the tape's positions must stay 16-byte aligned
       return None
+    total = torch.cuda.get_device_properties(device).total_memory
+    if 4 * n <= total // 1024:
+      try:
+        return torch.empty(n, dtype=torch.float32, device=device)
+      except torch.OutOfMemoryError:
+        return None
     free, _ = torch.cuda.mem_get_info(device)
     if 4 * n > free // 4:
       return None

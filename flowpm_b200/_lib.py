@@ -7,6 +7,7 @@ code.  There is no CPU or PyTorch fallback.
 import ctypes
 import os
 
+import numpy as np
 import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -96,6 +97,12 @@ SIGNATURES = {
     'fpm_power_spectrum': (c_int, [c_void_p, c_int, c_int, c_int, c_int,
                                    P_double, c_double, c_double, c_int,
                                    c_void_p, c_void_p]),
+    'fpm_growth_ode': (c_int, [c_void_p, c_void_p, c_int, c_void_p,
+                               c_void_p]),
+    'fpm_nbody_coefficients': (c_int, [c_void_p, c_void_p, c_int, c_double,
+                                       c_double, c_void_p, c_int, c_void_p]),
+    'fpm_lpt_coefficients': (c_int, [c_void_p, c_void_p, c_int, c_double,
+                                     c_double, c_double, c_void_p]),
     'fpm_white_noise': (c_int, [c_void_p, c_int64, c_uint64, c_double,
                                 c_void_p]),
     'fpm_cic_paint_2d': (c_int, [c_void_p, c_int, c_int, c_int, c_void_p,
@@ -183,8 +190,11 @@ def ptr(t):
 
 
 def dvec(values):
-  arr = (ctypes.c_double * len(values))(*[float(v) for v in values])
-  return arr
+  """Host array of doubles as a C argument (a copy of ``values``)."""
+  if isinstance(values, np.ndarray):
+    # the pointer object keeps the copy alive
+    return np.array(values, dtype=np.float64).ctypes.data_as(P_double)
+  return (ctypes.c_double * len(values))(*[float(v) for v in values])
 
 
 def ivec(values):

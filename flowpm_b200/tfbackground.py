@@ -14,6 +14,8 @@ reference does (flowpm/tfbackground.py:631-647).
 """
 import numpy as np
 
+from . import _lib
+
 __all__ = [
     'fde', 'w', 'E', 'H', 'dfde', 'dEa', 'Omega_m_a', 'Omega_de_a', 'D1', 'D2',
     'D1f', 'D2f', 'f1', 'f2', 'Gf', 'Gf2', 'gf', 'gf2', 'maybe_compute_ODE',
@@ -78,17 +80,6 @@ def Omega_de_a(cosmo, a):
   return cosmo.Omega_de * np.power(a, fde(cosmo, a)) / E(cosmo, a)**2
 
 
-def _growth_rhs(cosmo, a, y):
-  """Right-hand side of the growth system for y = (D1, D1', D2, D2')."""
-  om = Omega_m_a(cosmo, a)
-  friction = Omega_de_a(cosmo, a) - 0.5 * om + 2.0
-  d1, d1f, d2, d2f = y[..., 0], y[..., 1], y[..., 2], y[..., 3]
-  dd1 = 1.5 * om * d1 / a**2 - (d1f / a) * friction
-  dd2 = 1.5 * om * d2 / a**2 - (d2f / a) * friction - 1.5 * (
-      om * d1**2) / a**2
-  return np.stack([d1f, dd1, d2f, dd2], axis=-1)
-
-
 def maybe_compute_ODE(cosmo, log10_amin=-2, steps=256):
   """Growth tables on a = logspace(log10_amin, 0, steps), normalised to 1 at
   a = 1, cached in ``cosmo._workspace`` (:631-647)."""
@@ -96,18 +87,11 @@ def maybe_compute_ODE(cosmo, log10_amin=-2, steps=256):
   if key in cosmo._workspace:
     return cosmo._workspace[key]
   a = np.logspace(log10_amin, 0.0, steps)
-  y = np.array([a[0], 1.0, -3.0 / 7 * a[0]**2, -6.0 / 7 * a[0]])
-  ys = [y]
-  for i in range(steps - 1):
-    t, dt = a[i], a[i + 1] - a[i]
-    k1 = _growth_rhs(cosmo, t, y)
-    k2 = _growth_rhs(cosmo, t + dt / 2.0, y + dt * k1 / 2.0)
-    k3 = _growth_rhs(cosmo, t + dt / 2.0, y + dt * k2 / 2.0)
-    k4 = _growth_rhs(cosmo, t + dt, y + dt * k3)
-    y = y + dt * (k1 + 2.0 * k2 + 2.0 * k3 + k4) / 6.0
-    ys.append(y)
-  res = np.stack(ys)
-  second = _growth_rhs(cosmo, a, res)
+  res, second = np.empty((steps, 4)), np.empty((steps, 4))
+  par = np.array([cosmo.Omega_m, cosmo.Omega_k, cosmo.Omega_de, cosmo.w0,
+                  cosmo.wa], dtype=np.float64)
+  _lib.call('fpm_growth_ode', par.ctypes.data, a.ctypes.data, steps,
+            res.ctypes.data, second.ctypes.data)
   cache = {
       'a': a,
       'D1': res[:, 0] / res[-1, 0],
@@ -116,7 +100,10 @@ def maybe_compute_ODE(cosmo, log10_amin=-2, steps=256):
       'D2f': res[:, 3] / res[-1, 2],
       'F1p': second[:, 1] / res[-1, 0],
       'F2p': second[:, 3] / res[-1, 2],
+      'cosmo': par,
   }
+  cache['table'] = np.stack([cache[k] for k in ('D1', 'D1f', 'D2', 'D2f',
+                                                'F1p', 'F2p')])
   cosmo._workspace[key] = cache
   return cache
 
@@ -208,23 +195,21 @@ def drift_factor(cosmo, ai, ac, af):
 def nbody_coefficients(cosmo, stages):
   """Per-step {kick_start, drift, kick_end} of the KDK loop of
   flowpm/tfpm.py:475-498 for ``len(stages) - 1`` steps, shape (steps, 3)."""
-  stages = [float(s) for s in stages]
+  stages = np.array([float(s) for s in stages], dtype=np.float64)
   out = np.zeros((max(len(stages) - 1, 0), 3))
-  for i in range(len(stages) - 1):
-    a0, a1 = stages[i], stages[i + 1]
-    ah = (a0 * a1)**0.5
-    out[i, 0] = kick_factor(cosmo, a0, a0, ah)
-    out[i, 1] = drift_factor(cosmo, a0, ah, a1)
-    out[i, 2] = kick_factor(cosmo, ah, a1, a1)
+  c = maybe_compute_ODE(cosmo)
+  _lib.call('fpm_nbody_coefficients', c['cosmo'].ctypes.data,
+            c['table'].ctypes.data, len(c['a']), c['a'][0], c['a'][-1],
+            stages.ctypes.data, len(stages), out.ctypes.data)
   return out
 
 
 def lpt_coefficients(cosmo, a):
   """{D1, D2, a^2 f1 E, a^2 f2 E, a^2 E gf / D1, a^2 E gf2 / D2} of
   flowpm/tfpm.py:168-177."""
-  a = float(a)
-  d1, d2, e = float(D1(cosmo, a)), float(D2(cosmo, a)), float(E(cosmo, a))
-  return np.array([
-      d1, d2, a**2 * float(f1(cosmo, a)) * e, a**2 * float(f2(cosmo, a)) * e,
-      a**2 * e * float(gf(cosmo, a)) / d1, a**2 * e * float(gf2(cosmo, a)) / d2
-  ])
+  out = np.empty(6)
+  c = maybe_compute_ODE(cosmo)
+  _lib.call('fpm_lpt_coefficients', c['cosmo'].ctypes.data,
+            c['table'].ctypes.data, len(c['a']), c['a'][0], c['a'][-1],
+            float(a), out.ctypes.data)
+  return out

@@ -300,7 +300,7 @@ def nbody(cosmo, state, stages, nc, pm_nc_factor=1,
   forward ((steps + 1) x B x (pm_nc_factor nc)^3 floats, fpm_nbody_set_tape),
   so the backward takes its force meshes from it instead of painting and
   solving again; None (default) stores it when that takes less than a
-  quarter of the free device memory.
+  quarter of the free device memory (or under 1/1024 of the device's).
 
   With ``pgdparams`` (one row (alpha, kl, ks) per step) the PGD
   correction moves the particles after every drift (flowpm/tfpm.py:487-488,

@@ -492,6 +492,28 @@ int fpm_power_spectrum(const float* field, int batch, int nx, int ny, int nz,
 int fpm_white_noise(float* out, int64_t n, uint64_t seed, double stddev,
                     void* stream);
 
+/* Background cosmology on the host, FP64 (flowpm/tfbackground.py:533-647);
+ * every pointer is a host pointer.  cosmo = {Omega_m, Omega_k, Omega_de, w0,
+ * wa}.
+ *
+ * fpm_growth_ode: the growth system y = (D1, D1', D2, D2') by classic RK4 on
+ * the n scale factors a (increasing) from its matter-dominated start at
+ * a[0], and its derivatives dy, each n x 4, not normalised. */
+int fpm_growth_ode(const double* cosmo, const double* a, int n, double* y,
+                   double* dy);
+/* {kick_start, drift, kick_end} of each of the nstages - 1 leapfrog steps
+ * across stages (flowpm/tfpm.py:475-498), out (nstages - 1) x 3.  table: the
+ * six columns D1, D1', D2, D2', D1'', D2'' (normalised at the last scale
+ * factor) of n values on a grid regular in ln a over [a0, a1], column by
+ * column. */
+int fpm_nbody_coefficients(const double* cosmo, const double* table, int n,
+                           double a0, double a1, const double* stages,
+                           int nstages, double* out);
+/* {D1, D2, a^2 f1 E, a^2 f2 E, a^2 E gf / D1, a^2 E gf2 / D2} at a
+ * (flowpm/tfpm.py:168-177) from the same table. */
+int fpm_lpt_coefficients(const double* cosmo, const double* table, int n,
+                         double a0, double a1, double a, double* out);
+
 /* 2-D CIC paint, flowpm/utils.py:94-160 cic_paint_2d: mesh (batch, nx, ny)
  * += the 4-neighbour CIC weights of part (batch, npart, 2) in mesh units,
  * times weight (batch, npart; NULL: 1), for the particles whose mask byte

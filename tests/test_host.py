@@ -242,3 +242,32 @@ def test_product_does_not_import_oracle():
         with open(os.path.join(dirpath, f)) as fh:
           src = fh.read()
         assert 'oracle' not in src, f
+
+
+@pytest.mark.parametrize('kw', [{}, ALT, dict(Omega_k=0.05, w0=-0.9, wa=0.2)])
+def test_native_prefactors(fpm, kw):
+  """Kick, drift and LPT prefactors of the library against the functions of
+  tfbackground they are made of: the same formulas in double, so equal to a
+  few ulps of the differences they take (G and D1 of neighbouring stages
+  cancel at most two digits over 40 steps)."""
+  c = fpm.cosmology.Planck15(**kw)
+  bg = fpm.tfbackground
+  for stages in ([0.1], [0.3, 0.3001], np.linspace(0.02, 1.0, 41)):
+    co = bg.nbody_coefficients(c, stages)
+    assert co.shape == (len(stages) - 1, 3)
+    for (a0, a1), row in zip(zip(stages[:-1], stages[1:]), co):
+      ah = (a0 * a1)**0.5
+      ref = [bg.kick_factor(c, a0, a0, ah), bg.drift_factor(c, a0, ah, a1),
+             bg.kick_factor(c, ah, a1, a1)]
+      # relative step of the differenced functions
+      assert_allclose(row, ref, rtol=1e-15 * 64 / np.log(a1 / a0))
+  a = 0.1
+  assert_allclose(
+      bg.lpt_coefficients(c, a),
+      [bg.D1(c, a), bg.D2(c, a), a**2 * bg.f1(c, a) * bg.E(c, a),
+       a**2 * bg.f2(c, a) * bg.E(c, a),
+       a**2 * bg.E(c, a) * bg.gf(c, a) / bg.D1(c, a),
+       a**2 * bg.E(c, a) * bg.gf2(c, a) / bg.D2(c, a)], rtol=1e-13)
+  lib = fpm._lib.lib
+  assert lib.fpm_growth_ode(None, None, 0, None, None) == 1
+  assert lib.fpm_nbody_coefficients(None, None, 0, 0.0, 1.0, None, 0, None) == 1
