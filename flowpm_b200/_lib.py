@@ -97,6 +97,12 @@ SIGNATURES = {
     'fpm_power_spectrum': (c_int, [c_void_p, c_int, c_int, c_int, c_int,
                                    P_double, c_double, c_double, c_int,
                                    c_void_p, c_void_p]),
+    'fpm_power_spectrum_work': (c_int, [c_int, c_int, c_int, c_int, c_int,
+                                        P_int64]),
+    'fpm_power_spectrum_ws': (c_int, [c_void_p, c_int, c_int, c_int, c_int,
+                                      P_double, c_double, c_double, c_int,
+                                      c_void_p, c_void_p, c_int64,
+                                      c_void_p]),
     'fpm_growth_ode': (c_int, [c_void_p, c_void_p, c_int, c_void_p,
                                c_void_p]),
     'fpm_nbody_coefficients': (c_int, [c_void_p, c_void_p, c_int, c_double,

@@ -487,6 +487,17 @@ int fpm_power_spectrum(const float* field, int batch, int nx, int ny, int nz,
                        const double* boxsize, double kmin, double dk,
                        int nedges, float* power, void* stream);
 
+/* fpm_power_spectrum without an allocation of its own (its two scratch
+ * arrays; a new cuFFT plan still allocates its work area): work is
+ * caller-owned device memory, 16-byte aligned, of at least the bytes that
+ * fpm_power_spectrum_work gives. */
+int fpm_power_spectrum_work(int batch, int nx, int ny, int nz, int nedges,
+                            int64_t* bytes);
+int fpm_power_spectrum_ws(const float* field, int batch, int nx, int ny,
+                          int nz, const double* boxsize, double kmin,
+                          double dk, int nedges, float* power, void* work,
+                          int64_t work_bytes, void* stream);
+
 /* Gaussian white noise alone: out[e] = stddev * N(0,1) for e < n with the
  * generator of fpm_linear_field (counter = element index). */
 int fpm_white_noise(float* out, int64_t n, uint64_t seed, double stddev,
