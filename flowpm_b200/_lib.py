@@ -197,7 +197,7 @@ def ptr(t):
 
 def dvec(values):
   """Host array of doubles as a C argument (a copy of ``values``)."""
-  if isinstance(values, np.ndarray):
+  if isinstance(values, np.ndarray) and values.size > 16:
     # the pointer object keeps the copy alive
     return np.array(values, dtype=np.float64).ctypes.data_as(P_double)
   return (ctypes.c_double * len(values))(*[float(v) for v in values])

@@ -354,8 +354,8 @@ k_step_binned(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
     const bool last = (a.it == Tn);
     const float ks = last ? 0.f : cf[a.it * 3 + 0];
     const float dr = last ? 0.f : cf[a.it * 3 + 1];
-    const float fac = a.ffac[s];
-    const float invb = 1.0f / (float)S.bf;
+    // force = readout * factor / pm_nc_factor (flowpm/tfpm.py:218, :356)
+    const float fac = a.ffac[s] * (1.0f / (float)S.bf);
     const int64_t mcells = (int64_t)S.mx * S.my * S.mz;
     float* m = a.rho + S.r_off;
     const unsigned t = (unsigned)(ch - S.ch_t);
@@ -384,10 +384,7 @@ k_step_binned(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
       const Cic8 c0 = cic8(cic_axis(x.x, S.mx), cic_axis(x.y, S.my),
                            cic_axis(x.z, S.mz), S.my, S.mz);
       float3 f = readout_cic8(a.fmesh + 3 * S.m_off, mcells, c0);
-      // force = readout * factor / pm_nc_factor (flowpm/tfpm.py:218, :356)
-      f.x = __fmul_rn(__fmul_rn(f.x, fac), invb);
-      f.y = __fmul_rn(__fmul_rn(f.y, fac), invb);
-      f.z = __fmul_rn(__fmul_rn(f.z, fac), invb);
+      f = make_float3(f.x * fac, f.y * fac, f.z * fac);
       if (a.it >= 1) p = axpy(p, ke, f);  // closing kick of step it-1
       if (a.ckpt && a.it % a.ckpt_every == 0) {
         float* o = a.ckpt + (int64_t)(a.it / a.ckpt_every) * 2 * a.total_np * 3;
@@ -485,8 +482,8 @@ k_step_sorted(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
     const bool last = (a.it == Tn);
     const float ks = last ? 0.f : cf[a.it * 3 + 0];
     const float dr = last ? 0.f : cf[a.it * 3 + 1];
-    const float fac = a.ffac[s];
-    const float invb = 1.0f / (float)S.bf;
+    // force = readout * factor / pm_nc_factor (flowpm/tfpm.py:218, :356)
+    const float fac = a.ffac[s] * (1.0f / (float)S.bf);
     const int64_t mcells = (int64_t)S.mx * S.my * S.mz;
     float* m = a.rho + S.r_off;
     const int64_t first = S.p_off + (ch - S.ch_p) * kChunk;
@@ -511,8 +508,8 @@ k_step_sorted(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
       }
       const int64_t g = S.p_off + site_local(S, qi, qj, qk);  // Lagrangian
       const float3 x = mesh_pos(S, qi, qj, qk, d);
-      const Axis ax0 = cic_axis(x.x, S.mx), ay0 = cic_axis(x.y, S.my),
-                 az0 = cic_axis(x.z, S.mz);
+      Axis ax0, ay0, az0;
+      cic_axes(x, S.mx, S.my, S.mz, ax0, ay0, az0);
       const Cic8 c0 = cic8(ax0, ay0, az0, S.my, S.mz);
       // re-sorted as it moves: the run of lanes in this cell claims its
       // slots now; the claim's latency overlaps the readout
@@ -529,10 +526,7 @@ k_step_sorted(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
       }
       float3 f = valid ? readout_cic8(a.fmesh + 3 * S.m_off, mcells, c0)
                        : make_float3(0.f, 0.f, 0.f);
-      // force = readout * factor / pm_nc_factor (flowpm/tfpm.py:218, :356)
-      f.x = __fmul_rn(__fmul_rn(f.x, fac), invb);
-      f.y = __fmul_rn(__fmul_rn(f.y, fac), invb);
-      f.z = __fmul_rn(__fmul_rn(f.z, fac), invb);
+      f = make_float3(f.x * fac, f.y * fac, f.z * fac);
       if (a.it >= 1) p = axpy(p, ke, f);  // closing kick of step it-1
       if (valid && a.ckpt && a.it % a.ckpt_every == 0) {
         float* o = a.ckpt + (int64_t)(a.it / a.ckpt_every) * 2 * a.total_np * 3;
@@ -576,8 +570,8 @@ k_step_sorted(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
       }
       if (valid && !finite3(xn.x, xn.y, xn.z))
         atomicOr(a.status, FPM_STATUS_NONFINITE_POS);
-      const Axis nx1 = cic_axis(xn.x, S.mx), ny1 = cic_axis(xn.y, S.my),
-                 nz1 = cic_axis(xn.z, S.mz);
+      Axis nx1, ny1, nz1;
+      cic_axes(xn, S.mx, S.my, S.mz, nx1, ny1, nz1);
       const Cic8 c1 = cic8(nx1, ny1, nz1, S.my, S.mz);
       // base cell of the deposit; a lane past the sim's end gets a key of
       // its own
@@ -593,11 +587,7 @@ k_step_sorted(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
                     (int32_t)run_length(hs, lane));
       }
       float w[8];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        w[2 * q] = __fmul_rn(c1.wxy[q], c1.wz0);
-        w[2 * q + 1] = __fmul_rn(c1.wxy[q], c1.wz1);
-      }
+      cic_weights(c1, w);
       const unsigned heads = __ballot_sync(0xffffffffu, head);
       if (heads != 0xffffffffu) {
         // segmented sums over runs of contiguous lanes with equal keys (a

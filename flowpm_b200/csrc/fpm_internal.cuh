@@ -15,14 +15,14 @@ constexpr int kNumSMs = 148;     // B200
 
 // Lattice blocks of the particle kernels: (kPlanes wi) x kBJ x kBK
 // particles, z fastest, wi (SimDev::wi) particles per thread, chosen per
-// simulation; one pass of the block's threads covers kPlanes x planes.
-// Measured on B200 with kBJ = 4 / 8 / 16 at equal particles per block:
-// k_step at 2 x 512^3 8.92 / 8.70 / 8.68 ms, at 128^3 88.1 / 84.7 / 84.0
-// us; k_adj_position 15.4 / 15.8 / 16.7 ms.
+// simulation; one pass of the block's threads covers kPlanes x planes.  A
+// warp is one row of 32 along z.  Measured on B200, rows of 16 / 32 (blocks
+// of 8 x 16 and 4 x 32): k_step at 128^3 61.0 / 59.5 us, 2 x 90 x 100 x 126
+// 62.3 / 58.7 us, 512^3 3.44 / 3.40 ms; k_adj_position at 128^3 123 / 120 us.
 #ifndef FPM_BJ
-#define FPM_BJ 8
+#define FPM_BJ 4
 #endif
-constexpr int kBJ = FPM_BJ, kBK = 16;
+constexpr int kBJ = FPM_BJ, kBK = 32;
 constexpr int kPlanes = kThreads / (kBJ * kBK);
 static_assert(kPlanes * kBJ * kBK == kThreads, "whole x planes per pass");
 
@@ -217,6 +217,38 @@ __device__ __forceinline__ Axis cic_axis(float x, int n) {
   return a;
 }
 
+// cic_axis without a branch for |x| < 2^22 and a cell within one box length
+// of the mesh; false (the result void) for any other x.
+__device__ __forceinline__ bool cic_axis_near(float x, int n, Axis& a) {
+  const float r = __fadd_rn(x, kMagic);
+  int c = __float_as_int(r) - kMagicBits;
+  float f = __fsub_rn(r, kMagic);
+  const bool up = f > x;
+  f = up ? __fsub_rn(f, 1.0f) : f;
+  c = up ? c - 1 : c;
+  a.w0 = __fsub_rn(1.0f, fabsf(__fsub_rn(x, f)));
+  a.w1 = __fsub_rn(1.0f, fabsf(__fsub_rn(x, __fadd_rn(f, 1.0f))));
+  c += c < 0 ? n : 0;
+  c -= c >= n ? n : 0;
+  a.i0 = c;
+  a.i1 = c + 1 == n ? 0 : c + 1;
+  return (fabsf(x) < 4194304.0f) & ((unsigned)c < (unsigned)n);
+}
+
+// The three axes of a position: one branch for the whole position, taken
+// only when an axis needs the general path (six branches per position, and
+// their reconvergence, were 40 of k_step's 530 instructions).
+__device__ __forceinline__ void cic_axes(float3 x, int mx, int my, int mz,
+                                         Axis& ax, Axis& ay, Axis& az) {
+  const bool bx = cic_axis_near(x.x, mx, ax), by = cic_axis_near(x.y, my, ay),
+             bz = cic_axis_near(x.z, mz, az);
+  if (!(bx & by & bz)) {
+    ax = cic_axis(x.x, mx);
+    ay = cic_axis(x.y, my);
+    az = cic_axis(x.z, mz);
+  }
+}
+
 // Weight of neighbour (cx, cy, cz): (wx * wy) * wz, as the reference's
 // kernel[..., 0] * kernel[..., 1] * kernel[..., 2].
 __device__ __forceinline__ float cic_w(const Axis& ax, const Axis& ay,
@@ -238,6 +270,29 @@ __host__ __device__ __forceinline__ int conn_y(int c) {
 }
 __host__ __device__ __forceinline__ int conn_z(int c) {
   return (c == 3 || c == 5 || c == 6 || c == 7) ? 1 : 0;
+}
+
+// Two floats in one 64-bit register, for the packed FP32 instructions of
+// sm_100 (one issue for both).
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
 }
 
 __device__ __forceinline__ void red_add(float* p, float v) {
@@ -494,15 +549,29 @@ __device__ __forceinline__ void paint_rows(float* __restrict__ m, int pairs,
   }
 }
 
+// The weights of the four rows, w[2 q], w[2 q + 1] as paint_rows takes them.
+__device__ __forceinline__ void cic_weights(const Cic8& c, float* w) {
+  const uint64_t wz = pack2(c.wz0, c.wz1);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float2 v = unpack2(mul2(pack2(c.wxy[q], c.wxy[q]), wz));
+    w[2 * q] = v.x;
+    w[2 * q + 1] = v.y;
+  }
+}
+
 __device__ __forceinline__ void paint8(float* __restrict__ m, int pairs,
                                        const Cic8& c) {
   float w[8];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    w[2 * q] = __fmul_rn(c.wxy[q], c.wz0);
-    w[2 * q + 1] = __fmul_rn(c.wxy[q], c.wz1);
-  }
+  cic_weights(c, w);
   paint_rows(m, pairs, c, w);
+}
+
+// The CIC neighbours of mesh position x in simulation S.
+__device__ __forceinline__ Cic8 cic8_at(const SimDev& S, float3 x) {
+  Axis ax, ay, az;
+  cic_axes(x, S.mx, S.my, S.mz, ax, ay, az);
+  return cic8(ax, ay, az, S.my, S.mz);
 }
 
 // Deposit s * W at the 8 neighbours.
@@ -514,26 +583,27 @@ __device__ __forceinline__ void paint_scaled(float* __restrict__ m, int mx,
 }
 
 // Readout of the three force components (planes f0, f0 + mcells,
-// f0 + 2 mcells) at the same 8 neighbours.
+// f0 + 2 mcells) at the same 8 neighbours: per component the two z
+// neighbours of each row side by side in packed multiply-adds, summed at the
+// end (the product and sum of each of the 24 values rounded separately, in
+// the reference's order, took 33 more instructions for the same error).
 __device__ __forceinline__ float3 readout_cic8(const float* __restrict__ f0,
                                                int64_t mcells,
                                                const Cic8& c) {
   const float* f1 = f0 + mcells;
   const float* f2 = f1 + mcells;
-  float r0 = 0.f, r1 = 0.f, r2 = 0.f;
+  const uint64_t wz = pack2(c.wz0, c.wz1);
+  uint64_t r0 = 0, r1 = 0, r2 = 0;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const unsigned o0 = c.row[q] + c.z0, o1 = c.row[q] + c.z1;
-    const float w0 = __fmul_rn(c.wxy[q], c.wz0);
-    const float w1 = __fmul_rn(c.wxy[q], c.wz1);
-    r0 = __fadd_rn(r0, __fmul_rn(__ldg(f0 + o0), w0));
-    r1 = __fadd_rn(r1, __fmul_rn(__ldg(f1 + o0), w0));
-    r2 = __fadd_rn(r2, __fmul_rn(__ldg(f2 + o0), w0));
-    r0 = __fadd_rn(r0, __fmul_rn(__ldg(f0 + o1), w1));
-    r1 = __fadd_rn(r1, __fmul_rn(__ldg(f1 + o1), w1));
-    r2 = __fadd_rn(r2, __fmul_rn(__ldg(f2 + o1), w1));
+    const uint64_t w = mul2(pack2(c.wxy[q], c.wxy[q]), wz);
+    r0 = fma2(pack2(__ldg(f0 + o0), __ldg(f0 + o1)), w, r0);
+    r1 = fma2(pack2(__ldg(f1 + o0), __ldg(f1 + o1)), w, r1);
+    r2 = fma2(pack2(__ldg(f2 + o0), __ldg(f2 + o1)), w, r2);
   }
-  return make_float3(r0, r1, r2);
+  const float2 a = unpack2(r0), b = unpack2(r1), d = unpack2(r2);
+  return make_float3(a.x + a.y, b.x + b.y, d.x + d.y);
 }
 
 __device__ __forceinline__ float3 ld3(const float* p, int64_t g) {
@@ -544,12 +614,11 @@ __device__ __forceinline__ void st3(float* p, int64_t g, float3 v) {
   p[3 * g + 1] = v.y;
   p[3 * g + 2] = v.z;
 }
-// a + s * b with the two roundings of the reference (update = fac * F,
-// state = state + update).
+// a + s * b, rounded once (the reference's update = fac * F, state = state +
+// update rounds twice).
 __device__ __forceinline__ float3 axpy(float3 a, float s, float3 b) {
-  return make_float3(__fadd_rn(a.x, __fmul_rn(s, b.x)),
-                     __fadd_rn(a.y, __fmul_rn(s, b.y)),
-                     __fadd_rn(a.z, __fmul_rn(s, b.z)));
+  return make_float3(__fmaf_rn(s, b.x, a.x), __fmaf_rn(s, b.y, a.y),
+                     __fmaf_rn(s, b.z, a.z));
 }
 
 __device__ __forceinline__ void mode_ijl(int64_t local, int ny, int nzh,

@@ -31,8 +31,7 @@ k_paint_lattice(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
       const float3 d = ld3(disp, S.p_off + local);
       const float3 x = mesh_pos(S, i, j, k, d);
       if (!finite3(x.x, x.y, x.z)) atomicOr(status, FPM_STATUS_NONFINITE_POS);
-      paint8(m, S.pairs, cic8(cic_axis(x.x, S.mx), cic_axis(x.y, S.my),
-                              cic_axis(x.z, S.mz), S.my, S.mz));
+      paint8(m, S.pairs, cic8_at(S, x));
     }
   }
 }
@@ -51,8 +50,8 @@ k_step(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
     const bool last = (a.it == T);
     const float ks = last ? 0.f : cf[a.it * 3 + 0];
     const float dr = last ? 0.f : cf[a.it * 3 + 1];
-    const float fac = a.ffac[s];
-    const float invb = 1.0f / (float)S.bf;
+    // force = readout * factor / pm_nc_factor (flowpm/tfpm.py:218, :356)
+    const float fac = a.ffac[s] * (1.0f / (float)S.bf);
     const int64_t mcells = (int64_t)S.mx * S.my * S.mz;
     float* m = a.rho + S.r_off;
     const Walk w = walk_chunk(S, ch - traverse_first(S));
@@ -69,14 +68,10 @@ k_step(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
         p = ld3(a.mom, g);
       }
       const float3 x = mesh_pos(S, i, j, k, d);
-      const Cic8 c0 = cic8(cic_axis(x.x, S.mx), cic_axis(x.y, S.my),
-                           cic_axis(x.z, S.mz), S.my, S.mz);
+      const Cic8 c0 = cic8_at(S, x);
       float3 f = valid ? readout_cic8(a.fmesh + 3 * S.m_off, mcells, c0)
                        : make_float3(0.f, 0.f, 0.f);
-      // force = readout * factor / pm_nc_factor (flowpm/tfpm.py:218, :356)
-      f.x = __fmul_rn(__fmul_rn(f.x, fac), invb);
-      f.y = __fmul_rn(__fmul_rn(f.y, fac), invb);
-      f.z = __fmul_rn(__fmul_rn(f.z, fac), invb);
+      f = make_float3(f.x * fac, f.y * fac, f.z * fac);
       if (a.it >= 1) p = axpy(p, ke, f);  // closing kick of step it-1
       if (valid && a.ckpt && a.it % a.ckpt_every == 0) {
         float* o = a.ckpt + (int64_t)(a.it / a.ckpt_every) * 2 * a.total_np * 3;
@@ -110,8 +105,7 @@ k_step(const SimDev* __restrict__ sims, int nsims, int64_t ch0,
       const float3 xn = mesh_pos(S, i, j, k, d);
       if (valid && !finite3(xn.x, xn.y, xn.z))
         atomicOr(a.status, FPM_STATUS_NONFINITE_POS);
-      const Cic8 c1 = cic8(cic_axis(xn.x, S.mx), cic_axis(xn.y, S.my),
-                           cic_axis(xn.z, S.mz), S.my, S.mz);
+      const Cic8 c1 = cic8_at(S, xn);
       if (valid) paint8(m, S.pairs, c1);
     }
   }
@@ -148,17 +142,14 @@ k_pgd(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
       float3 d = ld3(disp, g);
       const float3 x = mesh_pos(S, i, j, k, d);
       const float3 r = readout_cic8(fmesh + 3 * S.m_off, mcells,
-                                    cic8(cic_axis(x.x, S.mx),
-                                         cic_axis(x.y, S.my),
-                                         cic_axis(x.z, S.mz), S.my, S.mz));
+                                    cic8_at(S, x));
       d.x = __fadd_rn(d.x, __fdiv_rn(__fmul_rn(r.x, alpha), b));
       d.y = __fadd_rn(d.y, __fdiv_rn(__fmul_rn(r.y, alpha), b));
       d.z = __fadd_rn(d.z, __fdiv_rn(__fmul_rn(r.z, alpha), b));
       st3(disp, g, d);
       const float3 xn = mesh_pos(S, i, j, k, d);
       if (!finite3(xn.x, xn.y, xn.z)) atomicOr(status, FPM_STATUS_NONFINITE_POS);
-      paint8(m, S.pairs, cic8(cic_axis(xn.x, S.mx), cic_axis(xn.y, S.my),
-                              cic_axis(xn.z, S.mz), S.my, S.mz));
+      paint8(m, S.pairs, cic8_at(S, xn));
     }
   }
 }
@@ -183,8 +174,7 @@ k_force_readout(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
       const float3 x = mesh_pos(S, i, j, k, ld3(disp, g));
       float3 f = readout_cic8(
           fmesh + 3 * S.m_off, mcells,
-          cic8(cic_axis(x.x, S.mx), cic_axis(x.y, S.my), cic_axis(x.z, S.mz),
-               S.my, S.mz));
+          cic8_at(S, x));
       f.x = __fmul_rn(__fmul_rn(f.x, fac), invb);
       f.y = __fmul_rn(__fmul_rn(f.y, fac), invb);
       f.z = __fmul_rn(__fmul_rn(f.z, fac), invb);

@@ -736,10 +736,13 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
     // at 2 x 512^3: k_step 9.14 / 8.90 / 8.73 / 8.70 ms and the reverse
     // position 18.1 / 17.5 / 17.3 / 17.1 ms at wi = 4 / 8 / 16 / 32; at
     // 128^3 wi = 4 is best (k_step 85 / 87 / 97 us at 4 / 8 / 16), larger
-    // blocks leaving too few of them for the SMs
+    // blocks leaving too few of them for the SMs.  Below 2^18 particles a
+    // thread takes one: at 32^3 (k_step 7.7 -> 3.7 us) four in a row were a
+    // serial chain on 32 of 148 SMs; 64^3 takes 11.2 us either way
     S.wi = (flags & FPM_PLAN_SMALL_BLOCKS) ? 4
            : S.np >= ((int64_t)1 << 26) ? FPM_WALK_LARGE
-           : S.np >= ((int64_t)1 << 23) ? 8 : 4;
+           : S.np >= ((int64_t)1 << 23) ? 8
+           : S.np >= ((int64_t)1 << 18) ? 4 : 1;
     S.nbi = (S.nx + kPlanes * S.wi - 1) / (kPlanes * S.wi);
     S.nbj = (S.ny + kBJ - 1) / kBJ;
     S.nbk = (S.nz + kBK - 1) / kBK;

@@ -66,10 +66,11 @@ enum {
                                     128 cells (powers of two) per axis use
                                     the library's fused Fourier solve       */
   FPM_PLAN_SMALL_BLOCKS = 1u << 5 /* the particle kernels walk every lattice
-                                    in blocks of 8x8x16 particles; by
+                                    in blocks of 8x4x32 particles; by
                                     default lattices of 2^23 particles or
-                                    more take 16x8x16 blocks, and of 2^26 or
-                                    more 64x8x16 (faster there)             */
+                                    more take 16x4x32 blocks, of 2^26 or
+                                    more 64x4x32, and below 2^18 2x4x32
+                                    (faster there)                          */
 };
 
 /* nbody flags (fpm_nbody). */
