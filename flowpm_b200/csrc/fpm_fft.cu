@@ -3,15 +3,16 @@
 // without cuFFT and without intermediate passes over HBM.
 //
 //   k_fft_plane_fwd  (one CTA per x plane)  rho(x, y, z) -> S(x, ky, kz)
-//       real-to-complex DFT along z, complex DFT along y, the plane held in
-//       shared memory; also zeroes rho for the next paint.
-//   k_fft_columns    (one CTA per group of (ky, kz) columns)
-//       DFT along x, then per component d the force spectrum
-//       F_d = S * pre * w(k) * i g_d (the transfer function of
-//       flowpm/tfpm.py:199-215 apply_longrange, the same arithmetic as
-//       k_fourier_force), inverse DFT along x -> F_d(x, ky, kz).
-//   k_fft_plane_inv  (one CTA per x plane and component)
-//       inverse DFT along y, complex-to-real along z -> force mesh d.
+//       real-to-complex DFT along z, complex DFT along y; also zeroes rho
+//       for the next paint.
+//   k_fft_x          (one CTA per 16 (ky, kz) columns)
+//       DFT along x, the transfer function (flowpm/tfpm.py:199-215
+//       apply_longrange), inverse DFT along x; also for meshes of 256 or 512
+//       along x.  k_fft_x_grad3: with the order-0 gradient, the three force
+//       spectra instead of the potential.
+//   k_fft_plane_inv  (one CTA per x plane, and component for order 0)
+//       inverse DFT along y, complex-to-real along z, y and z components of
+//       the force by the stencil; k_fft_stencil_x takes the x component.
 //
 // The transforms are unnormalised in both directions, as cuFFT's, so the
 // spectra have cuFFT's R2C layout (x, y, z/2 + 1) and the results match
@@ -32,8 +33,8 @@ namespace {
 constexpr int kFftThreads = 256;
 
 __constant__ float2 c_w128[128];  // exp(-2 pi i m / 128), m = 0..127
-__device__ float2 g_w128[128];    // the same, for lane-dependent indices
-__device__ float2 g_w512[512];    // exp(-2 pi i m / 512), m = 0..511
+__constant__ float2 c_w512[512];  // exp(-2 pi i m / 512), m = 0..511
+__device__ float2 g_w512[512];    // the same, for lane-dependent indices
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -65,10 +66,16 @@ template <>
 struct Split<128> {
   static constexpr int N1 = 16, N2 = 8;
 };
+template <>
+struct Split<256> {
+  static constexpr int N1 = 16, N2 = 16;
+};
+template <>
+struct Split<512> {
+  static constexpr int N1 = 32, N2 = 16;
+};
 
-// In-register radix-2 DFT of N (<= 16) values, decimation in time:
-// forward X[k] = sum_j x[j] exp(-2 pi i jk / N), inverse with +i.
-// In-register DFT of N (2 to 16) values by even/odd (radix-2, decimation
+// In-register DFT of N (2 to 32) values by even/odd (radix-2, decimation
 // in time) recursion, every index a compile-time constant: forward
 // X[k] = sum_j x[j] exp(-2 pi i jk / N), inverse with +i.
 template <int N, bool INV>
@@ -109,48 +116,113 @@ __device__ __forceinline__ void dft(float2 (&a)[N]) {
   Dft<N, INV>::run(a);
 }
 
-// Forward DFT of one line of N values by the N2 threads g of its group;
-// `line` (element e at line[e * es]) is the exchange buffer.  Every thread
-// of the block calls it; invalid threads (valid = false) get an in-bounds
-// line to read and write nothing.
-// On entry a[j1] = x[N2 j1 + g]; on exit a[u N2 + k2] = X[g + N2 u + N1 k2].
-// The caller syncs before writing the results back into `line`.
-template <int N>
-__device__ __forceinline__ void fwd_line(float2 (&a)[Split<N>::N1],
-                                         float2* line, int es, int g,
-                                         bool valid) {
-  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-  dft<N1, false>(a);
+// ---------------------------------------------------------------------------
+// Rows of real values, a group of N2 lanes per row (M complex values)
+// ---------------------------------------------------------------------------
+
+// Twiddles of a lane's row transform: t[k1] = W_M^(g k1) and w[e] =
+// W_2M^(k) of its element e = u N2 + k2, k = g + N2 u + N1 k2.
+template <int M>
+struct RowTw {
+  static constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2;
+  float2 t[N1], w[N1];
+  __device__ __forceinline__ void load(int g) {
 #pragma unroll
-  for (int k1 = 1; k1 < N1; ++k1)
-    a[k1] = cmul(a[k1], c_w128[((g * k1) & (N - 1)) * (128 / N)]);
-  __syncthreads();  // every line has been loaded
-  if (valid) {
+    for (int k1 = 0; k1 < N1; ++k1)
+      t[k1] = __ldg(&g_w512[((g * k1) & (M - 1)) * (512 / M)]);
 #pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) line[(k1 * N2 + g) * es] = a[k1];
+    for (int u = 0; u < N1 / N2; ++u)
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2)
+        w[u * N2 + k2] = __ldg(&g_w512[(g + N2 * u + N1 * k2) * (256 / M)]);
   }
-  __syncthreads();
+};
+
+// Slot of (k1, j) in a row's exchange: lanes of a group write one k1 at
+// consecutive j and read consecutive k1 at one j; the exclusive or spreads
+// the latter over the banks.
+template <int N2>
+__device__ __forceinline__ int ex_slot(int k1, int j) {
+  return k1 * N2 + (j ^ (k1 & (N2 - 1)));
+}
+
+// Element (u, k2) of the lane that holds M - k for this lane's k = g + N2 u
+// + N1 k2, fetched from it (lane g = 0 is its own partner).
+template <int M>
+__device__ __forceinline__ void row_partner(
+    const float2 (&a)[Split<M>::N1], int g, int lane,
+    float2 (&m)[Split<M>::N1]) {
+  constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2, U = N1 / N2;
+  const int src = (lane & ~(N2 - 1)) | ((N2 - g) & (N2 - 1));
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) {
+      const float2 v = a[(U - 1 - u) * N2 + (N2 - 1 - k2)];
+      const float2 t = make_float2(__shfl_sync(0xffffffffu, v.x, src),
+                                   __shfl_sync(0xffffffffu, v.y, src));
+      const float2 own = u == 0 ? a[(N2 - k2) & (N2 - 1)]
+                                : a[(U - u) * N2 + (N2 - 1 - k2)];
+      m[u * N2 + k2] = g ? t : own;
+    }
+}
+
+// Real-to-complex DFT of a row: on entry a[j1] = x[2m] + i x[2m + 1] of
+// element m = N2 j1 + g; on exit a[u N2 + k2] = X[k], k = g + N2 u + N1 k2,
+// except X[0], which is X[0] + i X[M] (both real).  X[k] = E + W_2M^k O with
+// E = (Z[k] + conj Z[M-k]) / 2 and O = (Z[k] - conj Z[M-k]) / 2i.  ex: M
+// slots of shared memory of the row's own; every lane of the warp takes
+// part.
+template <int M>
+__device__ __forceinline__ void row_r2c(float2 (&a)[Split<M>::N1], float2* ex,
+                                        int g, int lane, const RowTw<M>& tw) {
+  constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2;
+  dft<N1, false>(a);
+  __syncwarp();  // the row's slots are free
+#pragma unroll
+  for (int k1 = 0; k1 < N1; ++k1)
+    ex[ex_slot<N2>(k1, g)] = k1 ? cmul(a[k1], tw.t[k1]) : a[0];
+  __syncwarp();
 #pragma unroll
   for (int u = 0; u < N1 / N2; ++u) {
-    const int k1 = g + N2 * u;
     float2 b[N2];
 #pragma unroll
-    for (int j = 0; j < N2; ++j)
-      b[j] = line[(k1 * N2 + j) * es];
+    for (int j = 0; j < N2; ++j) b[j] = ex[ex_slot<N2>(g + N2 * u, j)];
     dft<N2, false>(b);
 #pragma unroll
     for (int k2 = 0; k2 < N2; ++k2) a[u * N2 + k2] = b[k2];
   }
+  float2 m[N1];
+  row_partner<M>(a, g, lane, m);
+#pragma unroll
+  for (int e = 0; e < N1; ++e) {
+    const float2 zk = a[e], zm = m[e];
+    const float2 E = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+    const float2 O = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
+    const float2 W = cmul(tw.w[e], O);
+    a[e] = make_float2(E.x + W.x, E.y + W.y);
+    if (e == 0 && g == 0) a[e] = make_float2(zk.x + zk.y, zk.x - zk.y);
+  }
 }
 
-// Inverse (unnormalised) DFT of one line, the converse of fwd_line:
-// on entry a[u N2 + k2] = X[g + N2 u + N1 k2]; on exit a[j1] = x[N2 j1 + g].
-template <int N>
-__device__ __forceinline__ void inv_line(float2 (&a)[Split<N>::N1],
-                                         float2* line, int es, int g,
-                                         bool valid) {
-  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-  __syncthreads();  // every line has been loaded
+// The converse (unnormalised): on entry a[u N2 + k2] = X[k] with X[0] + i
+// X[M] in the place of X[0]; on exit a[j1] = x[2m] + i x[2m + 1].
+template <int M>
+__device__ __forceinline__ void row_c2r(float2 (&a)[Split<M>::N1], float2* ex,
+                                        int g, int lane, const RowTw<M>& tw) {
+  constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2;
+  float2 m[N1];
+  row_partner<M>(a, g, lane, m);
+#pragma unroll
+  for (int e = 0; e < N1; ++e) {
+    const float2 xk = a[e], xm = m[e];
+    const float2 A = make_float2(xk.x + xm.x, xk.y - xm.y);
+    const float2 B = make_float2(xk.x - xm.x, xk.y + xm.y);
+    const float2 cb = cmulc(B, tw.w[e]);
+    a[e] = make_float2(A.x - cb.y, A.y + cb.x);  // A + i conj(W^k) B
+    if (e == 0 && g == 0) a[e] = make_float2(xk.x + xk.y, xk.x - xk.y);
+  }
+  __syncwarp();  // the row's slots are free
 #pragma unroll
   for (int u = 0; u < N1 / N2; ++u) {
     const int k1 = g + N2 * u;
@@ -159,418 +231,68 @@ __device__ __forceinline__ void inv_line(float2 (&a)[Split<N>::N1],
     for (int k2 = 0; k2 < N2; ++k2) b[k2] = a[u * N2 + k2];
     dft<N2, true>(b);
 #pragma unroll
-    for (int j2 = 0; j2 < N2; ++j2) {
-      if (j2 != 0 && k1 != 0)
-        b[j2] = cmulc(b[j2], c_w128[((j2 * k1) & (N - 1)) * (128 / N)]);
-      if (valid) line[(k1 * N2 + j2) * es] = b[j2];
-    }
+    for (int j2 = 0; j2 < N2; ++j2) ex[ex_slot<N2>(k1, j2)] = b[j2];
   }
-  __syncthreads();
+  __syncwarp();
 #pragma unroll
-  for (int k1 = 0; k1 < N1; ++k1)
-    a[k1] = line[(k1 * N2 + g) * es];
+  for (int k1 = 0; k1 < N1; ++k1) {
+    const float2 v = ex[ex_slot<N2>(k1, g)];
+    a[k1] = k1 ? cmulc(v, tw.t[k1]) : v;
+  }
   dft<N1, true>(a);
 }
 
-// Forward DFT along the rows (stride 1, length N, row stride rs) of
-// `nrows` rows of the shared plane P, in place, natural order out.
-template <int N, int T>
-__device__ __forceinline__ void rows_fwd(float2* P, int nrows, int rs) {
-  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-  constexpr int RP = T / N2;  // rows per pass (>= 32: warp-uniform g)
-  const int rl = threadIdx.x % RP, g = threadIdx.x / RP;
-#pragma unroll 1
-  for (int r0 = 0; r0 < nrows; r0 += RP) {
-    const int r = r0 + rl;
-    const bool valid = r < nrows;
-    float2* line = P + (valid ? r : 0) * rs;  // idle threads read row 0
-    float2 a[N1];
-#pragma unroll
-    for (int j1 = 0; j1 < N1; ++j1)
-      a[j1] = valid ? line[N2 * j1 + g] : make_float2(0.f, 0.f);
-    fwd_line<N>(a, line, 1, g, valid);
-    __syncthreads();
-    if (valid) {
-#pragma unroll
-      for (int u = 0; u < N1 / N2; ++u)
-#pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2)
-          line[g + N2 * u + N1 * k2] = a[u * N2 + k2];
-    }
-    __syncthreads();
-  }
+// The element before (element m - 1 of the row, periodic) of each element of
+// the lane, and the one after: v[j1] of lane g is element N2 j1 + g.
+template <int N1, int N2>
+__device__ __forceinline__ float row_prev(const float (&v)[N1], int j1, int g,
+                                          int lane) {
+  const float s = g == N2 - 1 ? v[(j1 + N1 - 1) % N1] : v[j1];
+  return __shfl_sync(0xffffffffu, s,
+                     (lane & ~(N2 - 1)) | ((g + N2 - 1) & (N2 - 1)));
+}
+template <int N1, int N2>
+__device__ __forceinline__ float row_next(const float (&v)[N1], int j1, int g,
+                                          int lane) {
+  const float s = g == 0 ? v[(j1 + 1) % N1] : v[j1];
+  return __shfl_sync(0xffffffffu, s,
+                     (lane & ~(N2 - 1)) | ((g + 1) & (N2 - 1)));
 }
 
-// Inverse DFT along the rows, in place, natural order in and out.
-template <int N, int T>
-__device__ __forceinline__ void rows_inv(float2* P, int nrows, int rs) {
-  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-  constexpr int RP = T / N2;
-  const int rl = threadIdx.x % RP, g = threadIdx.x / RP;
-#pragma unroll 1
-  for (int r0 = 0; r0 < nrows; r0 += RP) {
-    const int r = r0 + rl;
-    const bool valid = r < nrows;
-    float2* line = P + (valid ? r : 0) * rs;  // idle threads read row 0
-    float2 a[N1];
-#pragma unroll
-    for (int u = 0; u < N1 / N2; ++u)
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2)
-        a[u * N2 + k2] =
-            valid ? line[g + N2 * u + N1 * k2] : make_float2(0.f, 0.f);
-    inv_line<N>(a, line, 1, g, valid);
-    __syncthreads();
-    if (valid) {
-#pragma unroll
-      for (int j1 = 0; j1 < N1; ++j1) line[N2 * j1 + g] = a[j1];
-    }
-    __syncthreads();
-  }
-}
-
-// Forward / inverse DFT along the first NCOLS columns (length N, stride CS)
-// of P, in place, in one pass: T / N2 >= NCOLS.
-template <int N, bool INV, int T, int NCOLS, int CS>
-__device__ __forceinline__ void cols_dft(float2* P) {
-  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-  constexpr int CP = T / N2;
-  static_assert(CP >= NCOLS, "one pass over the columns");
-  const int c = threadIdx.x % CP, g = threadIdx.x / CP;
-  const bool valid = c < NCOLS;
-  float2* line = P + (valid ? c : 0);  // idle threads read column 0
-  float2 a[N1];
-  if constexpr (!INV) {
-#pragma unroll
-    for (int j1 = 0; j1 < N1; ++j1)
-      a[j1] = line[(N2 * j1 + g) * CS];
-    fwd_line<N>(a, line, CS, g, valid);
-    __syncthreads();
-    if (valid) {
-#pragma unroll
-      for (int u = 0; u < N1 / N2; ++u)
-#pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2)
-          line[(g + N2 * u + N1 * k2) * CS] = a[u * N2 + k2];
-    }
-  } else {
-#pragma unroll
-    for (int u = 0; u < N1 / N2; ++u)
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2)
-        a[u * N2 + k2] = line[(g + N2 * u + N1 * k2) * CS];
-    inv_line<N>(a, line, CS, g, valid);
-    __syncthreads();
-    if (valid) {
-#pragma unroll
-      for (int j1 = 0; j1 < N1; ++j1) line[(N2 * j1 + g) * CS] = a[j1];
-    }
-  }
-  __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
-// Kernels
-// ---------------------------------------------------------------------------
-
-// One x plane of one simulation of the run: rho -> S.  The real rows of
-// 2M cells are read as M complex values z[m] = x[2m] + i x[2m+1]; after the
-// M-point DFT Z, X[k] = E[k] + W^k O[k] (W = exp(-2 pi i / 2M)) with
-// E[k] = (Z[k] + conj Z[M-k]) / 2 and O[k] = (Z[k] - conj Z[M-k]) / 2i.
-// The columns kz = 0 and kz = M are real: they go through the y DFT
-// together as column 0 = X[.][0] + i X[.][M] and are separated on the way
-// out (Y0 = (C[ky] + conj C[-ky]) / 2, YM = (C[ky] - conj C[-ky]) / 2i), so
-// the y pass covers M columns.
-// Measured on B200 at 128^3 (Fourier solve per step): 512 threads 51 us,
-// 1024 threads 52 us; splitting each plane over a cluster of two CTAs
-// (the y pass through distributed shared memory) 63 us.
-#ifndef FPM_PLANE_THREADS
-#define FPM_PLANE_THREADS 512
-#endif
-constexpr int kPlaneThreads = FPM_PLANE_THREADS;  // threads of the plane kernels
-
-//
-// PAIRS: rho holds the painted z pairs (paint_rows, two floats per cell)
-// and the density is formed as the plane is loaded, rho[z] = P[z].x +
-// P[z - 1].y: one float4 is a complex value's two pairs, the y before them
-// comes from the lane below (or, at a warp's or a row's start, a load).
-template <int NY, int M, bool PAIRS>
-__global__ void __launch_bounds__(kPlaneThreads)
-k_fft_plane_fwd(const SimDev* __restrict__ sims, int first, int nx,
-                float* __restrict__ rho, float2* __restrict__ dk,
-                int painted, int zero_rho) {
-  pdl_wait();  // the density painted before
-  extern __shared__ float2 P[];  // NY rows of M + 1
-  constexpr int T = kPlaneThreads;
-  constexpr int NZH = M + 1;
-  const int s = first + blockIdx.x / nx;
-  const int x = blockIdx.x % nx;
-  const SimDev& S = sims[s];
-  constexpr int NF = PAIRS ? 2 : 1;       // floats per cell
-  constexpr int NV = NF * NY * M / 2;     // float4 per plane
-  float* plane = rho + (painted ? S.r_off : S.m_off) +
-                 (int64_t)x * NY * NF * 2 * M;
-  float4* src = reinterpret_cast<float4*>(plane);
-  float2* dst = dk + S.s_off + (int64_t)x * NY * NZH;
+// One row loaded as the a[] of row_r2c from the painted density P (PAIRS: z
+// pairs, one float4 per element, see paint_rows) or a plain mesh; zero: the
+// row is cleared (a lane clears what it alone has read).
+template <int M, bool PAIRS>
+__device__ __forceinline__ void row_load(float2 (&a)[Split<M>::N1], float* P,
+                                         int zero, int g, int lane) {
+  constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2;
   if (PAIRS) {
-    static_assert(NV % 32 == 0, "whole warps");
-    const int lane = threadIdx.x & 31;
-#pragma unroll 8
-    for (int e = threadIdx.x; e < NV; e += T) {
-      const float4 v = src[e];
-      const int r = e / M, m = e % M;
-      float y = __shfl_up_sync(0xffffffffu, v.w, 1);
-      if (lane == 0 || m == 0)
-        y = plane[4 * (m ? e - 1 : e + M - 1) + 3];
-      P[r * NZH + m] = make_float2(__fadd_rn(v.x, y), __fadd_rn(v.z, v.y));
+    float4* p4 = reinterpret_cast<float4*>(P);
+    float4 v[N1];
+    float y[N1];
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) v[j1] = p4[N2 * j1 + g];
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) y[j1] = v[j1].w;
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1)
+      a[j1] = make_float2(
+          __fadd_rn(v[j1].x, row_prev<N1, N2>(y, j1, g, lane)),
+          __fadd_rn(v[j1].z, v[j1].y));
+    if (zero) {
+#pragma unroll
+      for (int j1 = 0; j1 < N1; ++j1)
+        p4[N2 * j1 + g] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   } else {
-#pragma unroll 8
-    for (int e = threadIdx.x; e < NV; e += T) {
-      const float4 v = src[e];
-      const int r = (2 * e) / M, m = (2 * e) % M;
-      P[r * NZH + m] = make_float2(v.x, v.y);
-      P[r * NZH + m + 1] = make_float2(v.z, v.w);
-    }
-  }
-  __syncthreads();  // the whole plane has been read
-  if (zero_rho) {
-    for (int e = threadIdx.x; e < NV; e += T)
-      src[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  rows_fwd<M, T>(P, NY, NZH);
-  // real-to-complex unpacking, one (k, M - k) pair per work item
-  constexpr int KP = M / 2 + 1;
-  for (int e = threadIdx.x; e < NY * KP; e += T) {
-    const int r = e / KP, k = e % KP;
-    float2* line = P + r * NZH;
-    if (k == 0) {
-      const float2 z = line[0];
-      line[0] = make_float2(z.x + z.y, z.x - z.y);  // X[0] + i X[M]
-    } else if (2 * k == M) {
-      const float2 z = line[k];
-      line[k] = make_float2(z.x, -z.y);
-    } else {
-      const float2 zk = line[k], zm = line[M - k];
-      const float2 E = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
-      const float2 O = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
-      const float2 W = cmul(__ldg(&g_w128[k * (64 / M)]), O);
-      line[k] = make_float2(E.x + W.x, E.y + W.y);
-      line[M - k] = make_float2(E.x - W.x, -(E.y - W.y));
-    }
-  }
-  __syncthreads();
-  cols_dft<NY, false, T, M, NZH>(P);
-  for (int e = threadIdx.x; e < NY * NZH; e += T) {
-    const int ky = e / NZH, kz = e - ky * NZH;
-    float2 v;
-    if (kz == 0 || kz == M) {
-      const float2 c = P[ky * NZH];
-      const float2 cm = P[((NY - ky) & (NY - 1)) * NZH];
-      v = kz == 0 ? make_float2(0.5f * (c.x + cm.x), 0.5f * (c.y - cm.y))
-                  : make_float2(0.5f * (c.y + cm.y), -0.5f * (c.x - cm.x));
-    } else {
-      v = P[e];
-    }
-    dst[e] = v;
-  }
-}
-
-// Columns (ky, kz) of the spectra of one simulation: DFT along x, the three
-// force spectra, inverse DFT along x.  C = 256 / N2 columns per CTA, lanes
-// on consecutive columns (coalesced; warp-uniform group index g).
-template <int NX, bool GRAD3>
-__global__ void __launch_bounds__(kFftThreads)
-k_fft_columns(const SimDev* __restrict__ sims, int first, int nblk,
-              float2* dk, float2* __restrict__ fk, AxisTabs tabs, Green G) {
-  pdl_wait();
-  constexpr int N1 = Split<NX>::N1, N2 = Split<NX>::N2;
-  constexpr int C = kFftThreads / N2;
-  __shared__ float2 ex[C * NX];
-  const int s = first + blockIdx.x / nblk;
-  const SimDev& S = sims[s];
-  const int ny = S.my, nzh = S.mzh;
-  const int ncols = ny * nzh;
-  const int cl = threadIdx.x % C, g = threadIdx.x / C;
-  const int c = (blockIdx.x % nblk) * C + cl;
-  const bool valid = c < ncols;
-  const int64_t nmodes = (int64_t)NX * ncols;
-  const float2* src = dk + S.s_off + c;
-  float2* line = ex + cl;
-  float2 a[N1];
+    float2* p2 = reinterpret_cast<float2*>(P);
 #pragma unroll
-  for (int j1 = 0; j1 < N1; ++j1)
-    a[j1] = valid ? src[(int64_t)(N2 * j1 + g) * ncols] : make_float2(0.f, 0.f);
-  fwd_line<NX>(a, line, C, g, valid);
-  // potential spectrum delta * pre * w(k), w the transfer function G
-  const int ky = valid ? c / nzh : 0;
-  const int kz = valid ? c - ky * nzh : 0;
-  const float pre = (float)((double)S.bf * S.bf * S.bf /
-                            ((double)S.mx * S.my * S.mz));
-  const double* kkx = tabs.kk + S.tab;
-  const double* kky = kkx + S.mx;
-  const double* kkz = kky + S.my;
-  const float* wx = tabs.win + S.tab;
-  const float* wy = wx + S.mx;
-  const float* wz = wy + S.my;
-  const float* gx = tabs.grad + S.tab;
-  const float* gy = gx + S.mx;
-  const float* gz = gy + S.my;
-  const double kyz = kky[ky] + kkz[kz];
-  const float wyv = wy[ky], wzv = wz[kz];
-#pragma unroll
-  for (int u = 0; u < N1 / N2; ++u)
-#pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2) {
-      const int kx = g + N2 * u + N1 * k2;
-      const float w = green_w(G, s, kkx[kx] + kyz, wx[kx], wyv, wzv);
-      float2 v = a[u * N2 + k2];
-      v.x = __fmul_rn(__fmul_rn(v.x, pre), w);
-      v.y = __fmul_rn(__fmul_rn(v.y, pre), w);
-      a[u * N2 + k2] = v;
-    }
-  if (!GRAD3) {  // potential only, in place
-    inv_line<NX>(a, line, C, g, valid);
-    if (valid) {
-      float2* o = dk + S.s_off + c;
+    for (int j1 = 0; j1 < N1; ++j1) a[j1] = p2[N2 * j1 + g];
+    if (zero) {
 #pragma unroll
       for (int j1 = 0; j1 < N1; ++j1)
-        o[(int64_t)(N2 * j1 + g) * ncols] = a[j1];
+        p2[N2 * j1 + g] = make_float2(0.f, 0.f);
     }
-    return;
-  }
-  const float gyv = gy[ky], gzv = gz[kz];
-#pragma unroll 1
-  for (int d = 0; d < 3; ++d) {
-    float2 b[N1];
-#pragma unroll
-    for (int u = 0; u < N1 / N2; ++u)
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) {
-        const int kx = g + N2 * u + N1 * k2;
-        const float gd = d == 0 ? gx[kx] : (d == 1 ? gyv : gzv);
-        const float2 v = a[u * N2 + k2];
-        b[u * N2 + k2] = make_float2(-__fmul_rn(v.y, gd), __fmul_rn(v.x, gd));
-      }
-    inv_line<NX>(b, line, C, g, valid);
-    if (valid) {
-      float2* o = fk + 3 * S.s_off + d * nmodes + c;
-#pragma unroll
-      for (int j1 = 0; j1 < N1; ++j1)
-        o[(int64_t)(N2 * j1 + g) * ncols] = b[j1];
-    }
-  }
-}
-
-// x pass of the Fourier solve of meshes with 256 or 512 cells along x,
-// between batched two-dimensional (y, z) transforms of cuFFT (the
-// spectrum in cuFFT's R2C layout (x, y, z/2 + 1), unnormalised):
-// out = inverse-DFT_x(pre * w(k) * DFT_x(in)) for the kXCols consecutive
-// (ky, kz) columns of one simulation held by the block (the potential of
-// k_fourier_potential, the same arithmetic per mode).  The x DFT of
-// length NX = R * 64 runs on the stride-R sub-lines x = R b + a as 64-point
-// DFTs (cols_dft), a twiddle W_NX^(a kb) and R-point DFTs in registers,
-// where the transfer function is applied and the inverse starts; the
-// column block moves through shared memory as rows of kXCols modes.  With
-// zero, the block also zeroes its share of that buffer: zmul floats per
-// cell of the sim (1: the painted density, from r_off; 4: the interleaved
-// adjoint force mesh).
-// Columns per x-pass block.  Measured on B200 at 2 x 512^3: 8 columns
-// (64-byte rows, 32 KB) 1.19 ms per pass, 16 (128-byte rows, 64 KB) 1.01
-// ms; a persistent variant with cp.async double buffering of 8-column
-// blocks took 1.53 ms.
-#ifndef FPM_XPASS_COLS
-#define FPM_XPASS_COLS 16
-#endif
-constexpr int kXThreads = 512, kXCols = FPM_XPASS_COLS;
-
-template <int NX>
-__global__ void __launch_bounds__(kXThreads)
-k_fft_xcols(const SimDev* __restrict__ sims, int first, int nblk,
-            const float2* in, float2* out, float* __restrict__ zero,
-            int zmul, AxisTabs tabs, Green G,
-            const int32_t* __restrict__ nsteps, int pos) {
-  constexpr int R = NX / 64, C = kXCols, T = kXThreads;
-  constexpr int NP = 64 * C / T;                  // (kb, column) pairs
-  constexpr int NS = R * C, NS1 = NS < 64 ? NS : 64;  // sub-lines per pass
-  static_assert(64 * C % T == 0 && NS % NS1 == 0, "block shape");
-  extern __shared__ __align__(16) float2 buf[];   // x of column c at x C + c
-  pdl_wait();  // the spectrum written before
-  const int s = first + blockIdx.x / nblk;
-  if (nsteps && pos > nsteps[s]) return;  // finished simulation
-  const int blk = blockIdx.x % nblk;
-  const SimDev& S = sims[s];
-  const int ncols = S.my * S.mzh;
-  const int c0 = blk * C;
-  const float4* src = reinterpret_cast<const float4*>(in + S.s_off + c0);
-  float4* dst = reinterpret_cast<float4*>(out + S.s_off + c0);
-  const int64_t rstride = ncols / 2;  // float4 per x plane
-  float4* b4 = reinterpret_cast<float4*>(buf);
-#pragma unroll
-  for (int i = 0; i < NX * C / 2 / T; ++i) {
-    const int e = threadIdx.x + i * T;
-    b4[e] = src[(int64_t)(e / (C / 2)) * rstride + e % (C / 2)];
-  }
-  if (zero) {  // this block's share, in float4
-    const int64_t q4 = (int64_t)zmul * S.mx * S.my * S.mz / 4;
-    const int64_t per = (q4 + nblk - 1) / nblk;
-    float4* r4 = reinterpret_cast<float4*>(
-        zero + (zmul == 1 ? S.r_off : zmul * S.m_off));
-    const int64_t e1 = min(q4, (blk + 1) * per);
-    for (int64_t e = blk * per + threadIdx.x; e < e1; e += T)
-      r4[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int h = 0; h < NS / NS1; ++h)  // each ends with a barrier
-    cols_dft<64, false, T, NS1, NS>(buf + h * NS1);
-  const float pre = (float)((double)S.bf * S.bf * S.bf /
-                            ((double)S.mx * S.my * S.mz));
-#pragma unroll 1
-  for (int pr = 0; pr < NP; ++pr) {
-  const int kb = (threadIdx.x + pr * T) / C, c = threadIdx.x % C;
-  float2 v[R];
-#pragma unroll
-  for (int a = 0; a < R; ++a) {
-    v[a] = buf[(R * kb + a) * C + c];
-    if (a != 0 && kb != 0)
-      v[a] = cmul(v[a], g_w512[(a * kb * (512 / NX)) & 511]);
-  }
-  dft<R, false>(v);  // v[ka] = X[kb + 64 ka]
-  const int j = c0 + c;
-  const int ky = j / S.mzh, kz = j - ky * S.mzh;
-  const double* kkx = tabs.kk + S.tab;
-  const double kyv = kkx[S.mx + ky], kzv = kkx[S.mx + S.my + kz];
-  const float* wx = tabs.win + S.tab;
-  // the CIC windows only enter with deconvolution
-  const float wyv = G.deconv ? wx[S.mx + ky] : 1.f;
-  const float wzv = G.deconv ? wx[S.mx + S.my + kz] : 1.f;
-#pragma unroll
-  for (int ka = 0; ka < R; ++ka) {
-    const int kx = kb + 64 * ka;
-    const float w = green_w(G, s, (kkx[kx] + kyv) + kzv,
-                            G.deconv ? wx[kx] : 1.f, wyv, wzv);
-    float2 d = v[ka];
-    d.x = __fmul_rn(d.x, pre);
-    d.y = __fmul_rn(d.y, pre);
-    v[ka] = make_float2(__fmul_rn(d.x, w), __fmul_rn(d.y, w));
-  }
-  dft<R, true>(v);  // v[a] = sum_ka X W_R^(-a ka)
-#pragma unroll
-  for (int a = 0; a < R; ++a) {
-    if (a != 0 && kb != 0)
-      v[a] = cmulc(v[a], g_w512[(a * kb * (512 / NX)) & 511]);
-    buf[(R * kb + a) * C + c] = v[a];  // the positions this thread read
-  }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int h = 0; h < NS / NS1; ++h)
-    cols_dft<64, true, T, NS1, NS>(buf + h * NS1);
-#pragma unroll
-  for (int i = 0; i < NX * C / 2 / T; ++i) {
-    const int e = threadIdx.x + i * T;
-    dst[(int64_t)(e / (C / 2)) * rstride + e % (C / 2)] = b4[e];
   }
 }
 
@@ -583,11 +305,351 @@ __device__ __forceinline__ float stencil4f(float m2, float m1, float p1,
                    1.0f / 12.0f);
 }
 
-// One x plane of one force component: inverse DFT along y, then
-// complex-to-real along z: Zc[k] = A + i conj(W^k) B with A = X[k] +
-// conj X[M-k], B = X[k] - conj X[M-k], and the inverse M-point DFT of Zc
-// gives x[2m] + i x[2m+1].  The columns kz = 0 and kz = M, real after the y
-// inverse, share one complex column (X[.][0] + i X[.][M]).
+// z component of the 4-point gradient of the lane's elements (x[2m], x[2m +
+// 1]) of a row.
+template <int N1, int N2>
+__device__ __forceinline__ void row_grad(const float2 (&a)[N1],
+                                         float2 (&f)[N1], int g, int lane) {
+  float x[N1], y[N1];
+#pragma unroll
+  for (int j = 0; j < N1; ++j) {
+    x[j] = a[j].x;
+    y[j] = a[j].y;
+  }
+#pragma unroll
+  for (int j = 0; j < N1; ++j) {
+    const float px = row_prev<N1, N2>(x, j, g, lane),
+                py = row_prev<N1, N2>(y, j, g, lane),
+                nx = row_next<N1, N2>(x, j, g, lane),
+                ny = row_next<N1, N2>(y, j, g, lane);
+    f[j] = make_float2(stencil4f(px, py, y[j], nx),
+                       stencil4f(py, x[j], nx, ny));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Columns, N2 threads per column, each holding N1 values
+// ---------------------------------------------------------------------------
+
+// First half of a forward DFT of N values by thread g of its column: on
+// entry a[j1] = x[N2 j1 + g]; the N1-point DFTs, the twiddle and the write
+// to the exchange ex (slot q of the column at ex[q * cs]).
+template <int N>
+__device__ __forceinline__ void col_fwd_put(float2 (&a)[Split<N>::N1],
+                                            float2* ex, int cs, int g) {
+  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
+  dft<N1, false>(a);
+#pragma unroll
+  for (int k1 = 0; k1 < N1; ++k1)
+    ex[(k1 * N2 + g) * cs] =
+        k1 ? cmul(a[k1], c_w512[((g * k1) & (N - 1)) * (512 / N)]) : a[0];
+}
+// Second half, after a barrier: b[k2] = X[g + N2 u + N1 k2].  The slots read
+// are this thread's alone.
+template <int N>
+__device__ __forceinline__ void col_fwd_get(float2 (&b)[Split<N>::N2],
+                                            const float2* ex, int cs, int g,
+                                            int u) {
+  constexpr int N2 = Split<N>::N2;
+#pragma unroll
+  for (int j = 0; j < N2; ++j) b[j] = ex[((g + N2 * u) * N2 + j) * cs];
+  dft<N2, false>(b);
+}
+// The converse (unnormalised): b[k2] = X[g + N2 u + N1 k2] into this
+// thread's slots; after a barrier, a[j1] = x[N2 j1 + g].
+template <int N>
+__device__ __forceinline__ void col_inv_put(float2 (&b)[Split<N>::N2],
+                                            float2* ex, int cs, int g, int u) {
+  constexpr int N2 = Split<N>::N2;
+  const int k1 = g + N2 * u;
+  dft<N2, true>(b);
+#pragma unroll
+  for (int j2 = 0; j2 < N2; ++j2)
+    ex[(k1 * N2 + j2) * cs] =
+        j2 ? cmulc(b[j2], c_w512[((j2 * k1) & (N - 1)) * (512 / N)]) : b[0];
+}
+template <int N>
+__device__ __forceinline__ void col_inv_get(float2 (&a)[Split<N>::N1],
+                                            const float2* ex, int cs, int g) {
+  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
+#pragma unroll
+  for (int k1 = 0; k1 < N1; ++k1) a[k1] = ex[(k1 * N2 + g) * cs];
+  dft<N1, true>(a);
+}
+
+// ---------------------------------------------------------------------------
+// Kernels
+// ---------------------------------------------------------------------------
+
+// Threads of the plane kernels: one per column and exchange group, at least
+// four warps for the rows.
+template <int NY, int M>
+__host__ __device__ constexpr int plane_threads() {
+  return M * Split<NY>::N2 > 128 ? M * Split<NY>::N2 : 128;
+}
+// Row pitch of the plane in shared memory (float2): the rows that a half
+// warp touches together fall on different banks, and rows stay 16-byte
+// aligned.
+template <int M>
+__host__ __device__ constexpr int plane_pitch() {
+  return M + 8;
+}
+template <int NY, int M>
+__host__ __device__ constexpr size_t plane_smem() {
+  return (size_t)NY * (plane_pitch<M>() + M) * sizeof(float2);
+}
+
+// One x plane of one simulation of the run: rho -> S.  A warp transforms
+// 32 / N2 rows at a time from global memory in registers (exchanges within
+// the warp), then the block transforms the M columns (kz = 0 and kz = M are
+// real and go through the y DFT together as column 0 = X[.][0] + i X[.][M],
+// separated on the way out: Y0 = (C[ky] + conj C[-ky]) / 2, YM = (C[ky] -
+// conj C[-ky]) / 2i), one exchange through shared memory, results straight
+// to global memory.  Three block barriers; the same transform with the plane
+// in shared memory between every stage and a barrier around each took 14.6
+// us at 128^3 (25 MB read or cleared, 8 MB written, all in L2); this 10.5, the
+// inverse 13.7 and 11.0.  zero_rho: clears rho for the next paint.
+template <int NY, int M, bool PAIRS>
+__global__ void __launch_bounds__(plane_threads<NY, M>())
+k_fft_plane_fwd(const SimDev* __restrict__ sims, int first, int nx,
+                float* __restrict__ rho, float2* __restrict__ dk,
+                int painted, int zero_rho) {
+  extern __shared__ __align__(16) float2 smem[];
+  constexpr int T = plane_threads<NY, M>(), PP = plane_pitch<M>();
+  constexpr int R1 = Split<M>::N1, R2 = Split<M>::N2, RW = 32 / R2;
+  constexpr int N1 = Split<NY>::N1, N2 = Split<NY>::N2;
+  constexpr int NZH = M + 1;
+  float2* P = smem;            // NY rows of PP
+  float2* Q = smem + NY * PP;  // the columns' exchange
+  const int lane = threadIdx.x & 31, g = lane % R2;
+  RowTw<M> tw;
+  tw.load(g);
+  pdl_wait();  // the density painted before
+  const int s = first + blockIdx.x / nx;
+  const int x = blockIdx.x % nx;
+  const SimDev& S = sims[s];
+  constexpr int NF = PAIRS ? 2 : 1;  // floats per cell
+  float* plane = rho + (painted ? S.r_off : S.m_off) +
+                 (int64_t)x * NY * NF * 2 * M;
+  float2* dst = dk + S.s_off + (int64_t)x * NY * NZH;
+#pragma unroll 1
+  for (int r0 = (threadIdx.x >> 5) * RW; r0 < NY; r0 += T / 32 * RW) {
+    const int r = r0 + lane / R2;  // NY is a multiple of RW
+    float2 a[R1];
+    row_load<M, PAIRS>(a, plane + r * NF * 2 * M, zero_rho, g, lane);
+    float2* row = P + r * PP;
+    row_r2c<M>(a, row, g, lane, tw);
+    __syncwarp();  // the exchange has been read
+#pragma unroll
+    for (int u = 0; u < R1 / R2; ++u)
+#pragma unroll
+      for (int k2 = 0; k2 < R2; ++k2)
+        row[g + R2 * u + R1 * k2] = a[u * R2 + k2];
+  }
+  __syncthreads();
+  const int c = threadIdx.x % M, gc = threadIdx.x / M;
+  const bool col = T == M * N2 || gc < N2;
+  if (col) {
+    float2 a[N1];
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) a[j1] = P[(N2 * j1 + gc) * PP + c];
+    col_fwd_put<NY>(a, Q + c, M, gc);
+  }
+  __syncthreads();
+  float2* col0 = P;  // the plane has been read
+  if (col) {
+#pragma unroll
+    for (int u = 0; u < N1 / N2; ++u) {
+      float2 b[N2];
+      col_fwd_get<NY>(b, Q + c, M, gc, u);
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) {
+        const int ky = gc + N2 * u + N1 * k2;
+        if (c == 0)
+          col0[ky] = b[k2];
+        else
+          dst[ky * NZH + c] = b[k2];
+      }
+    }
+  }
+  __syncthreads();
+  for (int ky = threadIdx.x; ky < NY; ky += T) {
+    const float2 v = col0[ky], vm = col0[(NY - ky) & (NY - 1)];
+    dst[ky * NZH] = make_float2(0.5f * (v.x + vm.x), 0.5f * (v.y - vm.y));
+    dst[ky * NZH + M] = make_float2(0.5f * (v.y + vm.y), -0.5f * (v.x - vm.x));
+  }
+}
+
+// The x pass: out = inverse-DFT_x(pre * w(k) * DFT_x(in)) for kXCols
+// consecutive (ky, kz) columns of one simulation per block (spectra in the
+// R2C layout (x, y, z/2 + 1), unnormalised): the potential of
+// k_fourier_potential, the same arithmetic per mode.  N2 threads per column
+// hold N1 values each in registers from global memory and back, with one
+// exchange through shared memory each way: the slots that a thread reads
+// between the two are its own, so there are two barriers in all.  With zero,
+// the block also zeroes its share of that buffer: zmul floats per cell of the
+// sim (1: the painted density, from r_off; 4: the interleaved adjoint force
+// mesh).
+// Measured on B200 against a block that moved its columns through shared
+// memory in 64-point sub-lines (about 20 barriers) and divided in double:
+// 13.5 -> 7.2 us at 128^3, 0.47 -> 0.33 ms at 512^3 (1.08 GB, 3.2 TB/s), and
+// with the density's clearing 69 -> 47 us at 256^3.  The new exchange with the
+// double division took 13.0, 0.58 and 74: that division was the bound.
+constexpr int kXCols = 16;
+template <int NX>
+__host__ __device__ constexpr int x_threads() {
+  return kXCols * Split<NX>::N2;
+}
+
+// Blocks of the x pass that the registers of an SM hold.
+template <int NX>
+__host__ __device__ constexpr int x_blocks() {
+  return NX == 512 ? 2 : NX == 256 ? 3 : NX == 128 ? 6 : 8;
+}
+
+// PLAIN: the transfer function is the Green's function alone.
+template <int NX, bool PLAIN>
+__global__ void __launch_bounds__(x_threads<NX>(), x_blocks<NX>())
+k_fft_x(const SimDev* __restrict__ sims, int first, int nblk,
+        const float2* in, float2* out, float* __restrict__ zero, int zmul,
+        AxisTabs tabs, Green G, const int32_t* __restrict__ nsteps, int pos) {
+  constexpr int N1 = Split<NX>::N1, N2 = Split<NX>::N2, C = kXCols;
+  extern __shared__ __align__(16) float2 smem[];
+  pdl_wait();  // the spectrum written before
+  const int s = first + blockIdx.x / nblk;
+  if (nsteps && pos > nsteps[s]) return;  // finished simulation
+  const int blk = blockIdx.x % nblk;
+  const SimDev& S = sims[s];
+  const unsigned ncols = (unsigned)S.my * (unsigned)S.mzh;
+  const int cl = threadIdx.x % C, g = threadIdx.x / C;
+  const unsigned c = blk * C + cl;  // my is a multiple of 16
+  float2* ex = smem + cl;
+  const float2* src = in + S.s_off + c + (size_t)g * ncols;
+  float2 a[N1];
+#pragma unroll
+  for (int j1 = 0; j1 < N1; ++j1) a[j1] = src[(size_t)(N2 * j1) * ncols];
+  if (zero) {  // this block's share, in float4
+    const int64_t q4 = (int64_t)zmul * S.mx * S.my * S.mz / 4;
+    const int64_t per = (q4 + nblk - 1) / nblk;
+    float4* r4 = reinterpret_cast<float4*>(
+        zero + (zmul == 1 ? S.r_off : zmul * S.m_off));
+    const int64_t e1 = min(q4, (blk + 1) * per);
+    for (int64_t e = blk * per + threadIdx.x; e < e1; e += C * N2)
+      r4[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  // potential spectrum delta * pre * w(k), w the transfer function G
+  const unsigned ky = c / (unsigned)S.mzh, kz = c - ky * (unsigned)S.mzh;
+  const float pre = (float)((double)S.bf * S.bf * S.bf /
+                            ((double)S.mx * S.my * S.mz));
+  const double* kkx = tabs.kk + S.tab;
+  const float2* kk2 = tabs.kk2 + S.tab;
+  const float* wx = tabs.win + S.tab;
+  double kyz = 0.0;
+  float2 kyz2 = make_float2(0.f, 0.f);
+  float wyv = 1.f, wzv = 1.f;
+  if (PLAIN) {
+    kyz2 = two_add(kk2[S.mx + ky], kk2[S.mx + S.my + kz]);
+  } else {
+    kyz = kkx[S.mx + ky] + kkx[S.mx + S.my + kz];
+    // the CIC windows only enter with deconvolution
+    if (G.deconv) {
+      wyv = wx[S.mx + ky];
+      wzv = wx[S.mx + S.my + kz];
+    }
+  }
+  col_fwd_put<NX>(a, ex, C, g);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < N1 / N2; ++u) {
+    float2 b[N2];
+    col_fwd_get<NX>(b, ex, C, g, u);
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) {
+      const int kx = g + N2 * u + N1 * k2;
+      const float w =
+          PLAIN ? green_inv(kk2[kx], kyz2)
+                : green_w(G, s, kkx[kx] + kyz, G.deconv ? wx[kx] : 1.f, wyv,
+                          wzv);
+      b[k2].x = __fmul_rn(__fmul_rn(b[k2].x, pre), w);
+      b[k2].y = __fmul_rn(__fmul_rn(b[k2].y, pre), w);
+    }
+    col_inv_put<NX>(b, ex, C, g, u);
+  }
+  __syncthreads();
+  col_inv_get<NX>(a, ex, C, g);
+  float2* dst = out + S.s_off + c + (size_t)g * ncols;
+#pragma unroll
+  for (int j1 = 0; j1 < N1; ++j1) dst[(size_t)(N2 * j1) * ncols] = a[j1];
+}
+
+// Order-0 gradient: DFT along x, the three force spectra, inverse DFT along
+// x of each.
+template <int NX>
+__global__ void __launch_bounds__(x_threads<NX>())
+k_fft_x_grad3(const SimDev* __restrict__ sims, int first, int nblk,
+              const float2* __restrict__ dk, float2* __restrict__ fk,
+              AxisTabs tabs, Green G) {
+  constexpr int N1 = Split<NX>::N1, N2 = Split<NX>::N2, C = kXCols;
+  extern __shared__ __align__(16) float2 smem[];
+  pdl_wait();
+  const int s = first + blockIdx.x / nblk;
+  const SimDev& S = sims[s];
+  const unsigned ncols = (unsigned)S.my * (unsigned)S.mzh;
+  const int cl = threadIdx.x % C, g = threadIdx.x / C;
+  const unsigned c = (blockIdx.x % nblk) * C + cl;
+  const int64_t nmodes = (int64_t)NX * ncols;
+  float2* ex = smem + cl;
+  const float2* src = dk + S.s_off + c + (size_t)g * ncols;
+  float2 a[N1];
+#pragma unroll
+  for (int j1 = 0; j1 < N1; ++j1) a[j1] = src[(size_t)(N2 * j1) * ncols];
+  const unsigned ky = c / (unsigned)S.mzh, kz = c - ky * (unsigned)S.mzh;
+  const float pre = (float)((double)S.bf * S.bf * S.bf /
+                            ((double)S.mx * S.my * S.mz));
+  const double* kkx = tabs.kk + S.tab;
+  const double kyz = kkx[S.mx + ky] + kkx[S.mx + S.my + kz];
+  const float* wx = tabs.win + S.tab;
+  const float* gx = tabs.grad + S.tab;
+  const float gyv = gx[S.mx + ky], gzv = gx[S.mx + S.my + kz];
+  col_fwd_put<NX>(a, ex, C, g);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < N1 / N2; ++u) {
+    float2 b[N2];
+    col_fwd_get<NX>(b, ex, C, g, u);
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) {
+      const int kx = g + N2 * u + N1 * k2;
+      const float w = green_w(G, s, kkx[kx] + kyz, wx[kx], wx[S.mx + ky],
+                              wx[S.mx + S.my + kz]);
+      a[u * N2 + k2] = make_float2(__fmul_rn(__fmul_rn(b[k2].x, pre), w),
+                                   __fmul_rn(__fmul_rn(b[k2].y, pre), w));
+    }
+  }
+#pragma unroll 1
+  for (int d = 0; d < 3; ++d) {
+#pragma unroll
+    for (int u = 0; u < N1 / N2; ++u) {
+      float2 b[N2];
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) {
+        const int kx = g + N2 * u + N1 * k2;
+        const float gd = d == 0 ? gx[kx] : (d == 1 ? gyv : gzv);
+        const float2 v = a[u * N2 + k2];
+        b[k2] = make_float2(-__fmul_rn(v.y, gd), __fmul_rn(v.x, gd));
+      }
+      col_inv_put<NX>(b, ex, C, g, u);
+    }
+    __syncthreads();
+    float2 f[N1];
+    col_inv_get<NX>(f, ex, C, g);
+    __syncthreads();  // the next component overwrites the exchange
+    float2* o = fk + 3 * S.s_off + d * nmodes + c + (size_t)g * ncols;
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) o[(size_t)(N2 * j1) * ncols] = f[j1];
+  }
+}
+
 // Output modes of k_fft_plane_inv.
 enum PlaneOut {
   kOutStencil = 0,  // potential -> phi, force y and z by the 4-point stencil
@@ -595,16 +657,31 @@ enum PlaneOut {
   kOutReal = 2      // one spectrum -> one real mesh (phi)
 };
 
+// One x plane of one spectrum: inverse DFT along y from global memory (one
+// exchange), complex-to-real along z by warps in registers: Zc[k] = A + i
+// conj(W^k) B with A = X[k] + conj X[M-k], B = X[k] - conj X[M-k], and the
+// inverse M-point DFT of Zc gives x[2m] + i x[2m+1].  The columns kz = 0 and
+// kz = M, real after the y inverse, share one complex column (X[.][0] + i
+// X[.][M]).  With the stencil, the z component comes from the row in
+// registers, the y component from the plane in shared memory, each thread
+// walking along y with a window of five rows.
 template <int NY, int M, int MODE>
-__global__ void __launch_bounds__(kPlaneThreads)
+__global__ void __launch_bounds__(plane_threads<NY, M>())
 k_fft_plane_inv(const SimDev* __restrict__ sims, int first, int nx,
                 const float2* __restrict__ spec, float* __restrict__ fmesh,
                 float* __restrict__ phi) {
-  pdl_wait();
+  extern __shared__ __align__(16) float2 smem[];
   constexpr bool GRAD3 = MODE == kOutGrad3;
-  extern __shared__ float2 P[];
-  constexpr int T = kPlaneThreads;
+  constexpr int T = plane_threads<NY, M>(), PP = plane_pitch<M>();
+  constexpr int R1 = Split<M>::N1, R2 = Split<M>::N2, RW = 32 / R2;
+  constexpr int N1 = Split<NY>::N1, N2 = Split<NY>::N2;
   constexpr int NZH = M + 1;
+  float2* P = smem;
+  float2* Q = smem + NY * PP;
+  const int lane = threadIdx.x & 31, g = lane % R2;
+  RowTw<M> tw;
+  tw.load(g);
+  pdl_wait();
   const int d = GRAD3 ? blockIdx.x % 3 : 0;
   const int rest = GRAD3 ? blockIdx.x / 3 : blockIdx.x;
   const int x = rest % nx;
@@ -615,81 +692,83 @@ k_fft_plane_inv(const SimDev* __restrict__ sims, int first, int nx,
   const int64_t plane = (int64_t)x * NY * 2 * M;
   const float2* src = spec + (GRAD3 ? 3 * S.s_off + d * nmodes : S.s_off) +
                       (int64_t)x * NY * NZH;
-  // M columns per row after packing kz = 0 and kz = M into column 0
-  constexpr int NL = NY * M;
+  const int c = threadIdx.x % M, gc = threadIdx.x / M;
+  const bool col = T == M * N2 || gc < N2;
+  if (col) {
 #pragma unroll
-  for (int i = 0; i < (NL + T - 1) / T; ++i) {
-    const int e = threadIdx.x + i * T;
-    if (NL % T == 0 || e < NL) {
-      const int ky = e / M, kz = e % M;
-      const float2* row = src + ky * NZH;
-      float2 v = row[kz];
-      if (kz == 0) {
-        const float2 xm = row[M];
-        v = make_float2(v.x - xm.y, v.y + xm.x);
+    for (int u = 0; u < N1 / N2; ++u) {
+      float2 b[N2];
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) {
+        const float2* row = src + (gc + N2 * u + N1 * k2) * NZH;
+        b[k2] = row[c];
+        if (c == 0) {
+          const float2 xm = row[M];
+          b[k2] = make_float2(b[k2].x - xm.y, b[k2].y + xm.x);
+        }
       }
-      P[ky * NZH + kz] = v;
+      col_inv_put<NY>(b, Q + c, M, gc, u);
     }
   }
   __syncthreads();
-  cols_dft<NY, true, T, M, NZH>(P);
-  constexpr int KP = M / 2 + 1;
-  for (int e = threadIdx.x; e < NY * KP; e += T) {
-    const int r = e / KP, k = e % KP;
-    float2* line = P + r * NZH;
-    if (k == 0) {
-      const float2 c = line[0];  // X[0] + i X[M], both real
-      line[0] = make_float2(c.x + c.y, c.x - c.y);
-    } else if (2 * k == M) {
-      const float2 v = line[k];
-      line[k] = make_float2(2.f * v.x, -2.f * v.y);
-    } else {
-      const float2 xk = line[k], xm = line[M - k];
-      const float2 A = make_float2(xk.x + xm.x, xk.y - xm.y);
-      const float2 B = make_float2(xk.x - xm.x, xk.y + xm.y);
-      const float2 cb = cmulc(B, __ldg(&g_w128[k * (64 / M)]));
-      const float2 Tw = make_float2(-cb.y, cb.x);  // i conj(W^k) B
-      line[k] = make_float2(A.x + Tw.x, A.y + Tw.y);
-      line[M - k] = make_float2(A.x - Tw.x, -(A.y - Tw.y));
-    }
+  if (col) {
+    float2 a[N1];
+    col_inv_get<NY>(a, Q + c, M, gc);
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) P[(N2 * j1 + gc) * PP + c] = a[j1];
   }
   __syncthreads();
-  rows_inv<M, T>(P, NY, NZH);
-  constexpr int NV = NY * M / 2;  // float4 per plane
-  if (MODE != kOutStencil) {
-    float4* dst = reinterpret_cast<float4*>(
-        GRAD3 ? fmesh + 3 * S.m_off + d * mcells + plane
-              : phi + S.m_off + plane);
-    for (int e = threadIdx.x; e < NV; e += T) {
-      const int r = (2 * e) / M, m = (2 * e) % M;
-      const float2 a = P[r * NZH + m], b = P[r * NZH + m + 1];
-      dst[e] = make_float4(a.x, a.y, b.x, b.y);
+  float2* out = reinterpret_cast<float2*>(
+      GRAD3 ? fmesh + 3 * S.m_off + d * mcells + plane : phi + S.m_off + plane);
+  float2* fz = reinterpret_cast<float2*>(fmesh + 3 * S.m_off + 2 * mcells +
+                                         plane);
+#pragma unroll 1
+  for (int r0 = (threadIdx.x >> 5) * RW; r0 < NY; r0 += T / 32 * RW) {
+    const int r = r0 + lane / R2;
+    float2* row = P + r * PP;
+    float2 a[R1];
+#pragma unroll
+    for (int u = 0; u < R1 / R2; ++u)
+#pragma unroll
+      for (int k2 = 0; k2 < R2; ++k2)
+        a[u * R2 + k2] = row[g + R2 * u + R1 * k2];
+    row_c2r<M>(a, row, g, lane, tw);
+#pragma unroll
+    for (int j1 = 0; j1 < R1; ++j1) out[r * M + R2 * j1 + g] = a[j1];
+    if (MODE == kOutStencil) {
+      float2 f[R1];
+      row_grad<R1, R2>(a, f, g, lane);
+#pragma unroll
+      for (int j1 = 0; j1 < R1; ++j1) fz[r * M + R2 * j1 + g] = f[j1];
+      __syncwarp();  // the exchange has been read
+#pragma unroll
+      for (int j1 = 0; j1 < R1; ++j1) row[R2 * j1 + g] = a[j1];
     }
-    return;
   }
-  // potential plane: store it (the x stencil reads it) and take the y and
-  // z components of the force here, from shared memory
-  constexpr int RS = 2 * NZH;  // floats per row
-  constexpr int NZ = 2 * M;
-  const float* f = reinterpret_cast<const float*>(P);
-  float* gphi = phi + S.m_off + plane;
-  float* gy = fmesh + 3 * S.m_off + mcells + plane;
-  float* gz = fmesh + 3 * S.m_off + 2 * mcells + plane;
-  // consecutive lanes on consecutive z: conflict-free shared reads,
-  // coalesced stores
-  for (int e = threadIdx.x; e < NY * NZ; e += T) {
-    const int y = e / NZ, z = e % NZ;
-    const float* r0 = f + y * RS;
-    const float v = r0[z];
-    const float fy = stencil4f(f[((y - 2) & (NY - 1)) * RS + z],
-                               f[((y - 1) & (NY - 1)) * RS + z],
-                               f[((y + 1) & (NY - 1)) * RS + z],
-                               f[((y + 2) & (NY - 1)) * RS + z]);
-    const float fz = stencil4f(r0[(z - 2) & (NZ - 1)], r0[(z - 1) & (NZ - 1)],
-                               r0[(z + 1) & (NZ - 1)], r0[(z + 2) & (NZ - 1)]);
-    gphi[e] = v;
-    gy[e] = fy;
-    gz[e] = fz;
+  if (MODE != kOutStencil) return;
+  __syncthreads();
+  // y component: four z cells per thread, YL rows of them
+  constexpr int NQ = M / 2;                        // float4 per row
+  constexpr int NT = T / NQ < NY ? T / NQ : NY;    // threads along y
+  constexpr int YL = NY / NT;
+  const int q = threadIdx.x % NQ, t = threadIdx.x / NQ;
+  if (t >= NT) return;
+  float4* fy = reinterpret_cast<float4*>(fmesh + 3 * S.m_off + mcells + plane);
+  auto at = [&](int y) {
+    return reinterpret_cast<const float4*>(P + (y & (NY - 1)) * PP)[q];
+  };
+  const int y0 = t * YL;
+  float4 m2 = at(y0 - 2), m1 = at(y0 - 1), z = at(y0), p1 = at(y0 + 1);
+#pragma unroll
+  for (int i = 0; i < YL; ++i) {
+    const float4 p2 = at(y0 + i + 2);
+    fy[(y0 + i) * NQ + q] = make_float4(
+        stencil4f(m2.x, m1.x, p1.x, p2.x), stencil4f(m2.y, m1.y, p1.y, p2.y),
+        stencil4f(m2.z, m1.z, p1.z, p2.z), stencil4f(m2.w, m1.w, p1.w, p2.w));
+    m2 = m1;
+    m1 = z;
+    z = p1;
+    p1 = p2;
   }
 }
 
@@ -728,28 +807,30 @@ k_fft_stencil_x(const SimDev* __restrict__ sims, int first, int nx,
 std::mutex g_tw_mu;
 bool g_tw_ready[64] = {};
 
-template <int NY, int M>
-int set_plane_smem() {
-  const int bytes = NY * (M + 1) * (int)sizeof(float2);
-  if (cudaFuncSetAttribute(k_fft_plane_fwd<NY, M, true>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           bytes) != cudaSuccess ||
-      cudaFuncSetAttribute(k_fft_plane_fwd<NY, M, false>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           bytes) != cudaSuccess ||
-      cudaFuncSetAttribute(k_fft_plane_inv<NY, M, kOutStencil>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           bytes) != cudaSuccess ||
-      cudaFuncSetAttribute(k_fft_plane_inv<NY, M, kOutGrad3>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           bytes) != cudaSuccess ||
-      cudaFuncSetAttribute(k_fft_plane_inv<NY, M, kOutReal>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           bytes) != cudaSuccess) {
+int allow_smem(const void* k, size_t bytes) {
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)bytes) != cudaSuccess) {
     cudaGetLastError();
     return FPM_ERR_CUDA;
   }
   return FPM_OK;
+}
+
+template <int NY, int M>
+int set_plane_smem() {
+  constexpr size_t b = plane_smem<NY, M>();
+  for (const void* k : {(const void*)k_fft_plane_fwd<NY, M, true>,
+                        (const void*)k_fft_plane_fwd<NY, M, false>,
+                        (const void*)k_fft_plane_inv<NY, M, kOutStencil>,
+                        (const void*)k_fft_plane_inv<NY, M, kOutGrad3>,
+                        (const void*)k_fft_plane_inv<NY, M, kOutReal>})
+    if (allow_smem(k, b) != FPM_OK) return FPM_ERR_CUDA;
+  return FPM_OK;
+}
+
+template <int NX>
+__host__ __device__ constexpr size_t x_smem() {
+  return (size_t)NX * kXCols * sizeof(float2);
 }
 
 #define FPM_FFT_SIZES(X) X(16) X(32) X(64) X(128)
@@ -775,51 +856,43 @@ void launch_shape(const SimDev* sims, int first, int n, int nx, float* rho,
                   bool pairs, int zero_rho, float2* dk, float2* fk, float* fmesh,
                   float* phi, AxisTabs tabs, const Green& G, bool grad3,
                   bool real_out, cudaStream_t st) {
-  const size_t smem = (size_t)NY * (M + 1) * sizeof(float2);
+  constexpr size_t smem = plane_smem<NY, M>();
+  constexpr int T = plane_threads<NY, M>();
   auto fwd = pairs ? k_fft_plane_fwd<NY, M, true>
                    : k_fft_plane_fwd<NY, M, false>;
-  launch_pdl(fwd, dim3(n * nx), dim3(kPlaneThreads), smem, st, sims, first, nx,
-             rho, dk, real_out ? 0 : 1, zero_rho);
-  const int ncols = NY * (M + 1);
-  if (!grad3 && nx == 128) {
-    // x DFT, potential, inverse x DFT by the x-pass kernel (R = 2): four
-    // values per thread instead of sixteen, so more loads in flight
-    // (measured at 128^3: 47.7 against 48.7 us per Fourier solve)
-    const int nblk = ncols / kXCols;  // NY is a multiple of 16
-    launch_pdl(k_fft_xcols<128>, dim3(n * nblk), dim3(kXThreads),
-               (size_t)128 * kXCols * sizeof(float2), st, sims, first, nblk,
-               (const float2*)dk, dk, (float*)nullptr, 1, tabs, G,
-               (const int32_t*)nullptr, 0);
-  } else switch (nx) {
-#define FPM_COL_CASE(NN)                                                   \
-  case NN: {                                                               \
-    constexpr int C = kFftThreads / Split<NN>::N2;                         \
-    const int nblk = (ncols + C - 1) / C;                                  \
-    if (grad3)                                                             \
-      launch_pdl(k_fft_columns<NN, true>, dim3(n * nblk), dim3(kFftThreads), \
-                 0, st, sims, first, nblk, dk, fk, tabs, G);               \
-    else                                                                   \
-      launch_pdl(k_fft_columns<NN, false>, dim3(n * nblk),                 \
-                 dim3(kFftThreads), 0, st, sims, first, nblk, dk, fk, tabs, \
-                 G);                                                       \
-    break;                                                                 \
-  }
-    FPM_FFT_SIZES(FPM_COL_CASE)
-#undef FPM_COL_CASE
+  launch_pdl(fwd, dim3(n * nx), dim3(T), smem, st, sims, first, nx, rho, dk,
+             real_out ? 0 : 1, zero_rho);
+  const int nblk = NY * (M + 1) / kXCols;  // NY is a multiple of 16
+  const bool plain = green_plain(G);
+  switch (nx) {
+#define FPM_X_CASE(NN)                                                       \
+  case NN:                                                                   \
+    if (grad3)                                                               \
+      launch_pdl(k_fft_x_grad3<NN>, dim3(n * nblk), dim3(x_threads<NN>()),   \
+                 x_smem<NN>(), st, sims, first, nblk, (const float2*)dk, fk, \
+                 tabs, G);                                                   \
+    else                                                                     \
+      launch_pdl(plain ? k_fft_x<NN, true> : k_fft_x<NN, false>,             \
+                 dim3(n * nblk), dim3(x_threads<NN>()), x_smem<NN>(), st,    \
+                 sims, first, nblk, (const float2*)dk, dk,                   \
+                 (float*)nullptr, 1, tabs, G, (const int32_t*)nullptr, 0);   \
+    break;
+    FPM_FFT_SIZES(FPM_X_CASE)
+#undef FPM_X_CASE
   }
   if (grad3) {
-    k_fft_plane_inv<NY, M, kOutGrad3><<<n * nx * 3, kPlaneThreads, smem, st>>>(
+    k_fft_plane_inv<NY, M, kOutGrad3><<<n * nx * 3, T, smem, st>>>(
         sims, first, nx, fk, fmesh, phi);
     return;
   }
   if (real_out) {  // potential of `rho` -> phi
-    k_fft_plane_inv<NY, M, kOutReal><<<n * nx, kPlaneThreads, smem, st>>>(
+    k_fft_plane_inv<NY, M, kOutReal><<<n * nx, T, smem, st>>>(
         sims, first, nx, dk, nullptr, phi);
     return;
   }
   launch_pdl(k_fft_plane_inv<NY, M, kOutStencil>, dim3(n * nx),
-             dim3(kPlaneThreads), smem, st, sims, first, nx,
-             (const float2*)dk, fmesh, phi);
+             dim3(T), smem, st, sims, first, nx, (const float2*)dk, fmesh,
+             phi);
   const int64_t quads = (int64_t)nx * NY * 2 * M / 4;
   int64_t bx = (quads + kFftThreads - 1) / kFftThreads;
   const int64_t cap = (int64_t)kNumSMs * 8 / (n < 1 ? 1 : n) + 1;
@@ -851,30 +924,41 @@ bool fft_fused_supported(int nx, int ny, int nz) {
   return pow2_in_range(nx) && pow2_in_range(ny) && pow2_in_range(nz);
 }
 
-int fft_fused_prepare(int nx, int ny, int nz) {
-  if (!fft_fused_supported(nx, ny, nz)) return FPM_ERR_UNSUPPORTED;
+namespace {
+
+// Twiddle tables and shared-memory limits of the x pass, once per device.
+int prepare_device() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
     cudaGetLastError();
     return FPM_ERR_CUDA;
   }
-  {
-    std::lock_guard<std::mutex> lock(g_tw_mu);
-    if (!g_tw_ready[dev]) {
-      float2 w[128];
-      for (int m = 0; m < 128; ++m) {
-        const double t = -2.0 * 3.14159265358979323846 * m / 128.0;
-        w[m] = make_float2((float)std::cos(t), (float)std::sin(t));
-      }
-      if (cudaMemcpyToSymbol(c_w128, w, sizeof(w)) != cudaSuccess ||
-          cudaMemcpyToSymbol(g_w128, w, sizeof(w)) != cudaSuccess) {
-        cudaGetLastError();
-        return FPM_ERR_CUDA;
-      }
-      g_tw_ready[dev] = true;
-    }
+  std::lock_guard<std::mutex> lock(g_tw_mu);
+  if (g_tw_ready[dev]) return FPM_OK;
+  float2 w[512], w128[128];
+  for (int m = 0; m < 512; ++m) {
+    const double t = -2.0 * 3.14159265358979323846 * m / 512.0;
+    w[m] = make_float2((float)std::cos(t), (float)std::sin(t));
   }
-  if (nx == 128 && fft_xpass_prepare() != FPM_OK) return FPM_ERR_CUDA;
+  for (int m = 0; m < 128; ++m) w128[m] = w[4 * m];
+  if (cudaMemcpyToSymbol(c_w512, w, sizeof(w)) != cudaSuccess ||
+      cudaMemcpyToSymbol(g_w512, w, sizeof(w)) != cudaSuccess ||
+      cudaMemcpyToSymbol(c_w128, w128, sizeof(w128)) != cudaSuccess) {
+    cudaGetLastError();
+    return FPM_ERR_CUDA;
+  }
+  for (const void* k : {(const void*)k_fft_x<512, true>,
+                        (const void*)k_fft_x<512, false>})
+    if (allow_smem(k, x_smem<512>()) != FPM_OK) return FPM_ERR_CUDA;
+  g_tw_ready[dev] = true;
+  return FPM_OK;
+}
+
+}  // namespace
+
+int fft_fused_prepare(int nx, int ny, int nz) {
+  if (!fft_fused_supported(nx, ny, nz)) return FPM_ERR_UNSUPPORTED;
+  if (prepare_device() != FPM_OK) return FPM_ERR_CUDA;
   const int M = nz / 2;
   switch (ny) {
 #define FPM_PREP_CASE(NN) \
@@ -920,43 +1004,11 @@ void launch_fft_potential(const SimDev* sims, int first, int n, int nx,
   }
 }
 
-size_t xpass_smem(int nx) { return (size_t)nx * kXCols * sizeof(float2); }
-
 bool fft_xpass_supported(int nx, int ny, int nz) {
   return (nx == 256 || nx == 512) && ny % kXCols == 0 && nz % 2 == 0;
 }
 
-int fft_xpass_prepare() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-    cudaGetLastError();
-    return FPM_ERR_CUDA;
-  }
-  static bool ready[64] = {};
-  std::lock_guard<std::mutex> lock(g_tw_mu);
-  if (ready[dev]) return FPM_OK;
-  float2 w[512];
-  for (int m = 0; m < 512; ++m) {
-    const double t = -2.0 * 3.14159265358979323846 * m / 512.0;
-    w[m] = make_float2((float)std::cos(t), (float)std::sin(t));
-  }
-  float2 w128[128];
-  for (int m = 0; m < 128; ++m) w128[m] = w[4 * m];
-  if (cudaMemcpyToSymbol(g_w512, w, sizeof(w)) != cudaSuccess ||
-      cudaMemcpyToSymbol(c_w128, w128, sizeof(w128)) != cudaSuccess ||
-      cudaMemcpyToSymbol(g_w128, w128, sizeof(w128)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_fft_xcols<512>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)xpass_smem(512)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_fft_xcols<256>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)xpass_smem(256)) != cudaSuccess) {
-    cudaGetLastError();
-    return FPM_ERR_CUDA;
-  }
-  ready[dev] = true;
-  return FPM_OK;
-}
+int fft_xpass_prepare() { return prepare_device(); }
 
 void launch_fft_xpass(const SimDev* sims, int first, int n, int nx, int ny,
                       int nzh, const float2* in, float2* out, float* zero,
@@ -966,12 +1018,16 @@ void launch_fft_xpass(const SimDev* sims, int first, int n, int nx, int ny,
   g_launches.fetch_add(1, std::memory_order_relaxed);
   const int nblk = ny * nzh / kXCols;
   const unsigned grid = (unsigned)(n * nblk);
-  if (nx == 512)
-    k_fft_xcols<512><<<grid, kXThreads, xpass_smem(512), st>>>(
+  const bool plain = green_plain(G);
+  if (nx == 512) {
+    auto k = plain ? k_fft_x<512, true> : k_fft_x<512, false>;
+    k<<<grid, x_threads<512>(), x_smem<512>(), st>>>(
         sims, first, nblk, in, out, zero, zmul, tabs, G, nsteps, pos);
-  else
-    k_fft_xcols<256><<<grid, kXThreads, xpass_smem(256), st>>>(
+  } else {
+    auto k = plain ? k_fft_x<256, true> : k_fft_x<256, false>;
+    k<<<grid, x_threads<256>(), x_smem<256>(), st>>>(
         sims, first, nblk, in, out, zero, zmul, tabs, G, nsteps, pos);
+  }
 }
 
 }  // namespace fpm

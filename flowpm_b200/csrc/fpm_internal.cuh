@@ -68,9 +68,11 @@ struct SimDev {
 // k = 2*pi*fftfreq(i, n) (flowpm/kernels.py:10-25):
 //   kk  = k^2 (double), grad = (8 sin k - sin 2k)/6 (kernels.py:72-76) or
 //   k with the Nyquist entry zeroed (order 0, kernels.py:66-70),
-//   win = sinc(k / 2pi)^-2 (kernels.py:137-152).
+//   win = sinc(k / 2pi)^-2 (kernels.py:137-152); kk2 = kk as the sum of two
+//   floats (48 bits).
 struct AxisTabs {
   const double* kk;
+  const float2* kk2;
   const float* grad;
   const float* win;
 };
@@ -116,6 +118,31 @@ __device__ __forceinline__ float green_w(const Green& G, int s, double kk,
   if (G.r2 != 0.0) w = __fmul_rn(w, (float)exp(-kk * G.r2));
   if (G.deconv) w = __fmul_rn(w, __fmul_rn(__fmul_rn(wx, wy), wz));
   return w;
+}
+
+// Whether G is the Green's function alone.
+__host__ __device__ inline bool green_plain(const Green& G) {
+  return !G.pgd && G.r2 == 0.0 && !G.deconv;
+}
+
+// a + b of two-float values, the first sum exact (Knuth's two-sum).
+__device__ __forceinline__ float2 two_add(float2 a, float2 b) {
+  const float h = __fadd_rn(a.x, b.x);
+  const float t = __fsub_rn(h, a.x);
+  const float e = __fadd_rn(__fsub_rn(a.x, __fsub_rn(h, t)),
+                            __fsub_rn(b.x, t));
+  return make_float2(h, __fadd_rn(e, __fadd_rn(a.y, b.y)));
+}
+
+// 1 / kk rounded to float, kk = kx + kyz as two floats: an approximate
+// reciprocal and one Newton step on the full value (0 at k = 0).  In double
+// (one division per mode) the x pass was bound by it.
+__device__ __forceinline__ float green_inv(float2 kx, float2 kyz) {
+  const float2 kk = two_add(kx, kyz);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(kk.x));
+  const float e = __fmaf_rn(-kk.y, r, __fmaf_rn(-kk.x, r, 1.f));
+  return kk.x == 0.f ? 0.f : __fmaf_rn(r, e, r);
 }
 
 enum ChunkKind {

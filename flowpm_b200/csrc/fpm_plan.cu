@@ -83,6 +83,7 @@ struct fpm_plan {
   int64_t ch_p = 0, ch_s = 0, ch_m = 0, ch_l = 0, ch_ls = 0, ch_b = 0;
   // tables
   double* d_kk = nullptr;
+  float2* d_kk2 = nullptr;
   float* d_grad = nullptr;
   float* d_win = nullptr;
   // force-mesh buffers
@@ -166,7 +167,9 @@ struct fpm_plan {
 
 namespace {
 
-AxisTabs tabs_of(const fpm_plan* p) { return AxisTabs{p->d_kk, p->d_grad, p->d_win}; }
+AxisTabs tabs_of(const fpm_plan* p) {
+  return AxisTabs{p->d_kk, p->d_kk2, p->d_grad, p->d_win};
+}
 
 Green plan_green(const fpm_plan* p) {
   return force_green(p->r_split * p->r_split,
@@ -222,7 +225,7 @@ void free_all(fpm_plan* p) {
   if (p->ev_fork) cudaEventDestroy(p->ev_fork);
   for (int k = 0; k < kProfKinds; ++k)
     for (cudaEvent_t e : p->ev[k]) cudaEventDestroy(e);
-  void* bufs[] = {p->d_sims, p->d_kk,   p->d_grad,  p->d_win,   p->rho,
+  void* bufs[] = {p->d_sims, p->d_kk, p->d_kk2,   p->d_grad,  p->d_win,   p->rho,
                   p->dk,     p->fk,     p->fmesh,   p->lreal1,  p->lspec1,
                   p->lspec9, p->lreal9, p->lreal3,  p->d_coefs, p->d_nsteps,
                   p->d_ffac, p->d_lcoef, p->d_status, p->work, p->d_pgd,
@@ -890,6 +893,7 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
   size_t& tot = p->device_bytes;
   p->d_sims = dalloc<SimDev>(nsims, tot, ok);
   p->d_kk = dalloc<double>(kk.size(), tot, ok);
+  p->d_kk2 = dalloc<float2>(kk.size(), tot, ok);
   p->d_grad = dalloc<float>(grad.size(), tot, ok);
   p->d_win = dalloc<float>(win.size(), tot, ok);
   p->rho = dalloc<float>(p->total_r, tot, ok);
@@ -930,8 +934,15 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
     for (cufftHandle h : hs)
       if (h && cufftSetWorkArea(h, p->work) != CUFFT_SUCCESS) rc = FPM_ERR_CUFFT;
   }
+  std::vector<float2> kk2(kk.size());
+  for (size_t i = 0; i < kk.size(); ++i) {
+    kk2[i].x = (float)kk[i];
+    kk2[i].y = (float)(kk[i] - (double)kk2[i].x);
+  }
   if (rc == FPM_OK &&
-      (cudaMemcpy(p->d_sims, p->sims.data(), sizeof(SimDev) * nsims,
+      (cudaMemcpy(p->d_kk2, kk2.data(), sizeof(float2) * kk2.size(),
+                  cudaMemcpyHostToDevice) != cudaSuccess ||
+       cudaMemcpy(p->d_sims, p->sims.data(), sizeof(SimDev) * nsims,
                   cudaMemcpyHostToDevice) != cudaSuccess ||
        cudaMemcpy(p->d_kk, kk.data(), sizeof(double) * kk.size(),
                   cudaMemcpyHostToDevice) != cudaSuccess ||
