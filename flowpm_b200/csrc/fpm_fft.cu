@@ -122,19 +122,31 @@ __device__ __forceinline__ void dft(float2 (&a)[N]) {
 
 // Twiddles of a lane's row transform: t[k1] = W_M^(g k1) and w[e] =
 // W_2M^(k) of its element e = u N2 + k2, k = g + N2 u + N1 k2.
+//
+// Rows of more than 64 values would keep 64 registers of them: their w[e] is
+// read from the table where it is used.
 template <int M>
 struct RowTw {
   static constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2;
-  float2 t[N1], w[N1];
-  __device__ __forceinline__ void load(int g) {
+  static constexpr bool kKeep = M <= 64;
+  float2 t[N1], w[kKeep ? N1 : 1];
+  int g;
+  static __device__ __forceinline__ float2 table(int g, int e) {
+    const int k = g + N2 * (e / N2) + N1 * (e % N2);
+    return __ldg(&g_w512[k * (256 / M)]);
+  }
+  __device__ __forceinline__ void load(int lane_g) {
+    g = lane_g;
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1)
       t[k1] = __ldg(&g_w512[((g * k1) & (M - 1)) * (512 / M)]);
+    if (kKeep) {
 #pragma unroll
-    for (int u = 0; u < N1 / N2; ++u)
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2)
-        w[u * N2 + k2] = __ldg(&g_w512[(g + N2 * u + N1 * k2) * (256 / M)]);
+      for (int e = 0; e < N1; ++e) w[kKeep ? e : 0] = table(g, e);
+    }
+  }
+  __device__ __forceinline__ float2 at(int e) const {
+    return kKeep ? w[kKeep ? e : 0] : table(g, e);
   }
 };
 
@@ -199,7 +211,7 @@ __device__ __forceinline__ void row_r2c(float2 (&a)[Split<M>::N1], float2* ex,
     const float2 zk = a[e], zm = m[e];
     const float2 E = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
     const float2 O = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
-    const float2 W = cmul(tw.w[e], O);
+    const float2 W = cmul(tw.at(e), O);
     a[e] = make_float2(E.x + W.x, E.y + W.y);
     if (e == 0 && g == 0) a[e] = make_float2(zk.x + zk.y, zk.x - zk.y);
   }
@@ -218,7 +230,7 @@ __device__ __forceinline__ void row_c2r(float2 (&a)[Split<M>::N1], float2* ex,
     const float2 xk = a[e], xm = m[e];
     const float2 A = make_float2(xk.x + xm.x, xk.y - xm.y);
     const float2 B = make_float2(xk.x - xm.x, xk.y + xm.y);
-    const float2 cb = cmulc(B, tw.w[e]);
+    const float2 cb = cmulc(B, tw.at(e));
     a[e] = make_float2(A.x - cb.y, A.y + cb.x);  // A + i conj(W^k) B
     if (e == 0 && g == 0) a[e] = make_float2(xk.x + xk.y, xk.x - xk.y);
   }
@@ -650,6 +662,148 @@ k_fft_x_grad3(const SimDev* __restrict__ sims, int first, int nblk,
   }
 }
 
+// ---------------------------------------------------------------------------
+// z and y passes of meshes whose planes do not fit one block (ny and nz of
+// 256 or 512): rows along z by warps in registers, columns along y as the x
+// pass.  Each is one read and one write of the mesh or spectrum, the density
+// formed from its z pairs and cleared in the first, the z component of the
+// force taken in the last.  Measured against the library's plane transforms
+// with a kernel for the pairs before and the whole stencil after: at 512^3
+// 0.40 + 0.33 + 0.24 -> 0.41 + 0.27 ms forward, 0.24 + 0.34 + 0.41 -> 0.24 +
+// 0.28 + 0.29 ms back; at 256^3, 35 + 27 -> 33 + 30 us and 27 + 34 + 55 -> 30
+// + 42 + 41.  A plain density of 256^3 is better cleared by the x pass (6 us
+// there) than here: rows of 8 bytes a lane read and cleared in one pass took
+// 83 us.
+// ---------------------------------------------------------------------------
+constexpr int kZThreads = 256;
+
+template <int M, bool PAIRS>
+__global__ void __launch_bounds__(kZThreads, 2)
+k_fft_z_fwd(const SimDev* __restrict__ sims, int first, int nrows,
+            float* __restrict__ rho, float2* __restrict__ dk, int painted,
+            int zero, const int32_t* __restrict__ nsteps, int pos) {
+  constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2, RW = 32 / N2;
+  constexpr int PP = M + 8;  // rows of a half warp on different banks
+  __shared__ float2 ex_[kZThreads / N2][PP];
+  const int s = first + blockIdx.y;
+  if (nsteps && pos > nsteps[s]) return;  // finished simulation
+  const int lane = threadIdx.x & 31, g = lane % N2;
+  RowTw<M> tw;
+  tw.load(g);
+  constexpr int NF = PAIRS ? 2 : 1;
+  float* in = rho + (painted ? sims[s].r_off : sims[s].m_off);
+  float2* out = dk + sims[s].s_off;
+  float2* ex = ex_[threadIdx.x / N2];
+  const int wpb = kZThreads / 32;
+  for (int r0 = (blockIdx.x * wpb + (threadIdx.x >> 5)) * RW; r0 < nrows;
+       r0 += gridDim.x * wpb * RW) {  // nrows is a multiple of RW
+    const int r = r0 + lane / N2;
+    float2 a[N1];
+    row_load<M, PAIRS>(a, in + (size_t)r * NF * 2 * M, zero, g, lane);
+    row_r2c<M>(a, ex, g, lane, tw);
+    float2* o = out + (size_t)r * (M + 1);
+#pragma unroll
+    for (int e = 0; e < N1; ++e) {
+      float2 v = a[e];
+      if (e == 0 && g == 0) {  // X[0] and X[M], both real
+        o[M] = make_float2(v.y, 0.f);
+        v.y = 0.f;
+      }
+      o[g + N2 * (e / N2) + N1 * (e % N2)] = v;
+    }
+  }
+}
+
+// GRAD: also the z component of the force of each row.
+template <int M, bool GRAD>
+__global__ void __launch_bounds__(kZThreads, 2)
+k_fft_z_inv(const SimDev* __restrict__ sims, int first, int nrows,
+            const float2* __restrict__ spec, float* __restrict__ phi,
+            float* __restrict__ fmesh, const int32_t* __restrict__ nsteps,
+            int pos) {
+  constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2, RW = 32 / N2;
+  constexpr int PP = M + 8;
+  __shared__ float2 ex_[kZThreads / N2][PP];
+  const int s = first + blockIdx.y;
+  if (nsteps && pos > nsteps[s]) return;
+  const int lane = threadIdx.x & 31, g = lane % N2;
+  RowTw<M> tw;
+  tw.load(g);
+  const SimDev& S = sims[s];
+  const float2* in = spec + S.s_off;
+  float2* out = reinterpret_cast<float2*>(phi + S.m_off);
+  float2* fz = reinterpret_cast<float2*>(
+      fmesh + 3 * S.m_off + 2 * (int64_t)S.mx * S.my * S.mz);
+  float2* ex = ex_[threadIdx.x / N2];
+  const int wpb = kZThreads / 32;
+  for (int r0 = (blockIdx.x * wpb + (threadIdx.x >> 5)) * RW; r0 < nrows;
+       r0 += gridDim.x * wpb * RW) {
+    const int r = r0 + lane / N2;
+    const float2* x = in + (size_t)r * (M + 1);
+    float2 a[N1];
+#pragma unroll
+    for (int e = 0; e < N1; ++e) a[e] = x[g + N2 * (e / N2) + N1 * (e % N2)];
+    if (g == 0) a[0].y = x[M].x;  // both real
+    row_c2r<M>(a, ex, g, lane, tw);
+    const size_t o = (size_t)r * M + g;
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) out[o + N2 * j1] = a[j1];
+    if (GRAD) {
+      float2 f[N1];
+      row_grad<N1, N2>(a, f, g, lane);
+#pragma unroll
+      for (int j1 = 0; j1 < N1; ++j1) fz[o + N2 * j1] = f[j1];
+    }
+  }
+}
+
+// DFT along y of kXCols consecutive columns (x, kz) per block, in place.
+template <int NY, bool INV>
+__global__ void __launch_bounds__(x_threads<NY>(), x_blocks<NY>())
+k_fft_y(const SimDev* __restrict__ sims, int first, float2* __restrict__ dk,
+        const int32_t* __restrict__ nsteps, int pos) {
+  constexpr int N1 = Split<NY>::N1, N2 = Split<NY>::N2, C = kXCols;
+  extern __shared__ __align__(16) float2 smem[];
+  const int s = first + blockIdx.y;
+  if (nsteps && pos > nsteps[s]) return;
+  const SimDev& S = sims[s];
+  const unsigned nzh = S.mzh;
+  const int cl = threadIdx.x % C, g = threadIdx.x / C;
+  const unsigned q = blockIdx.x * C + cl;  // mx is a multiple of 16
+  const unsigned x = q / nzh, kz = q - x * nzh;
+  float2* col = dk + S.s_off + (size_t)x * NY * nzh + kz;
+  float2* ex = smem + cl;
+  if (!INV) {
+    float2 a[N1];
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) a[j1] = col[(N2 * j1 + g) * nzh];
+    col_fwd_put<NY>(a, ex, C, g);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < N1 / N2; ++u) {
+      float2 b[N2];
+      col_fwd_get<NY>(b, ex, C, g, u);
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2)
+        col[(g + N2 * u + N1 * k2) * nzh] = b[k2];
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < N1 / N2; ++u) {
+      float2 b[N2];
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2)
+        b[k2] = col[(g + N2 * u + N1 * k2) * nzh];
+      col_inv_put<NY>(b, ex, C, g, u);
+    }
+    __syncthreads();
+    float2 a[N1];
+    col_inv_get<NY>(a, ex, C, g);
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) col[(N2 * j1 + g) * nzh] = a[j1];
+  }
+}
+
 // Output modes of k_fft_plane_inv.
 enum PlaneOut {
   kOutStencil = 0,  // potential -> phi, force y and z by the 4-point stencil
@@ -948,7 +1102,9 @@ int prepare_device() {
     return FPM_ERR_CUDA;
   }
   for (const void* k : {(const void*)k_fft_x<512, true>,
-                        (const void*)k_fft_x<512, false>})
+                        (const void*)k_fft_x<512, false>,
+                        (const void*)k_fft_y<512, true>,
+                        (const void*)k_fft_y<512, false>})
     if (allow_smem(k, x_smem<512>()) != FPM_OK) return FPM_ERR_CUDA;
   g_tw_ready[dev] = true;
   return FPM_OK;
@@ -1028,6 +1184,62 @@ void launch_fft_xpass(const SimDev* sims, int first, int n, int nx, int ny,
     k<<<grid, x_threads<256>(), x_smem<256>(), st>>>(
         sims, first, nblk, in, out, zero, zmul, tabs, G, nsteps, pos);
   }
+}
+
+bool fft_zy_supported(int ny, int nz) {
+  return (ny == 256 || ny == 512) && (nz == 256 || nz == 512);
+}
+
+namespace {
+
+// Blocks of the row kernels: every SM full twice over.
+dim3 z_grid(int nx, int ny, int M, int n) {
+  const int rows = nx * ny, per = kZThreads / (M == 256 ? 16 : 8);
+  const int blocks = rows / per, cap = kNumSMs * 8;
+  return dim3((unsigned)(blocks < cap ? blocks : cap), (unsigned)n);
+}
+
+template <bool INV>
+void launch_y(const SimDev* sims, int first, int n, int nx, int ny, int nz,
+              float2* dk, const int32_t* nsteps, int pos, cudaStream_t st) {
+  const dim3 grid((unsigned)(nx * (nz / 2 + 1) / kXCols), (unsigned)n);
+  if (ny == 512)
+    k_fft_y<512, INV><<<grid, x_threads<512>(), x_smem<512>(), st>>>(
+        sims, first, dk, nsteps, pos);
+  else
+    k_fft_y<256, INV><<<grid, x_threads<256>(), x_smem<256>(), st>>>(
+        sims, first, dk, nsteps, pos);
+}
+
+}  // namespace
+
+void launch_fft_zy_fwd(const SimDev* sims, int first, int n, int nx, int ny,
+                       int nz, float* rho, bool painted, bool pairs, int zero,
+                       float2* dk, const int32_t* nsteps, int pos,
+                       cudaStream_t st) {
+  if (n <= 0) return;
+  g_launches.fetch_add(2, std::memory_order_relaxed);
+  const int M = nz / 2;
+  auto k = M == 256 ? (pairs ? k_fft_z_fwd<256, true> : k_fft_z_fwd<256, false>)
+                    : (pairs ? k_fft_z_fwd<128, true>
+                             : k_fft_z_fwd<128, false>);
+  k<<<z_grid(nx, ny, M, n), kZThreads, 0, st>>>(
+      sims, first, nx * ny, rho, dk, painted ? 1 : 0, zero, nsteps, pos);
+  launch_y<false>(sims, first, n, nx, ny, nz, dk, nsteps, pos, st);
+}
+
+void launch_fft_zy_inv(const SimDev* sims, int first, int n, int nx, int ny,
+                       int nz, float2* spec, float* phi, float* fmesh,
+                       const int32_t* nsteps, int pos, cudaStream_t st) {
+  if (n <= 0) return;
+  g_launches.fetch_add(2, std::memory_order_relaxed);
+  launch_y<true>(sims, first, n, nx, ny, nz, spec, nsteps, pos, st);
+  const int M = nz / 2;
+  auto k = M == 256 ? (fmesh ? k_fft_z_inv<256, true> : k_fft_z_inv<256, false>)
+                    : (fmesh ? k_fft_z_inv<128, true>
+                             : k_fft_z_inv<128, false>);
+  k<<<z_grid(nx, ny, M, n), kZThreads, 0, st>>>(sims, first, nx * ny, spec,
+                                                phi, fmesh, nsteps, pos);
 }
 
 }  // namespace fpm

@@ -1084,18 +1084,17 @@ void launch_stencil_div_tiled(const SimDev* sims, int first, int count,
 
 void launch_stencil_grad_tiled(const SimDev* sims, int first, int count,
                                int mx, int my, int mz, int xc,
-                               const float* phi, float* fmesh,
+                               const float* phi, float* fmesh, bool with_z,
                                const int32_t* nsteps, int pos,
                                cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   const dim3 grid((unsigned)((mx / xc) * (my / kDivTY) * (mz / kDivTZ)),
                   (unsigned)count);
-  if (xc == 32)
-    k_stencil_grad_tiled<32, true><<<grid, 256, 0, st>>>(sims, first, phi,
-                                                         fmesh, nsteps, pos);
-  else
-    k_stencil_grad_tiled<16, true><<<grid, 256, 0, st>>>(sims, first, phi,
-                                                         fmesh, nsteps, pos);
+  auto k = xc == 32 ? (with_z ? k_stencil_grad_tiled<32, true>
+                              : k_stencil_grad_tiled<32, false>)
+                    : (with_z ? k_stencil_grad_tiled<16, true>
+                              : k_stencil_grad_tiled<16, false>);
+  k<<<grid, 256, 0, st>>>(sims, first, phi, fmesh, nsteps, pos);
 }
 
 void launch_step(const SimDev* sims, int nsims, int64_t ch0, int64_t ch1,

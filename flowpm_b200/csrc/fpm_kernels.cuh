@@ -73,10 +73,11 @@ void launch_stencil_div(const SimDev* sims, int nsims, int64_t nchunks,
 // launch_stencil_div).
 int stencil_div_chunk(int mx, int my, int mz, int64_t m_off, int count);
 // Tiled k_stencil_grad (the same tiles and x chunk as the tiled
-// divergence) over the sims [first, first + count) of one mesh shape.
+// divergence) over the sims [first, first + count) of one mesh shape; with_z
+// false: the x and y components alone.
 void launch_stencil_grad_tiled(const SimDev* sims, int first, int count,
                                int mx, int my, int mz, int xc,
-                               const float* phi, float* fmesh,
+                               const float* phi, float* fmesh, bool with_z,
                                const int32_t* nsteps, int pos,
                                cudaStream_t st);
 void launch_stencil_div_tiled(const SimDev* sims, int first, int count,
@@ -122,6 +123,21 @@ void launch_fft_xpass(const SimDev* sims, int first, int n, int nx, int ny,
                       int nzh, const float2* in, float2* out, float* zero,
                       int zmul, AxisTabs tabs, const Green& G,
                       const int32_t* nsteps, int pos, cudaStream_t st);
+
+// The plane transforms around the x pass for ny and nz of 256 or 512.
+// Forward: R2C along z and DFT along y of the sims [first, first + n) of one
+// run into dk, from the painted density rho (painted; pairs: z pairs) or a
+// plain mesh; zero: clears what it reads.  Inverse: in place on spec, then
+// C2R along z into phi and, with fmesh, the z component of the 4-point
+// gradient into the third plane of each sim.
+bool fft_zy_supported(int ny, int nz);
+void launch_fft_zy_fwd(const SimDev* sims, int first, int n, int nx, int ny,
+                       int nz, float* rho, bool painted, bool pairs, int zero,
+                       float2* dk, const int32_t* nsteps, int pos,
+                       cudaStream_t st);
+void launch_fft_zy_inv(const SimDev* sims, int first, int n, int nx, int ny,
+                       int nz, float2* spec, float* phi, float* fmesh,
+                       const int32_t* nsteps, int pos, cudaStream_t st);
 
 // Fused readout + kick(end) + kick(start) + drift + paint of one iteration,
 // over the traversal chunks [ch0, ch1) (whole simulations).

@@ -43,6 +43,8 @@ struct Run {
   bool fused = false;      // force meshes by the fused Fourier solve
   bool xpass = false;      // r2c / c2r1 are batched (y, z) plane transforms
                            // around the x-pass kernel
+  bool zy = false;         // x pass with the library's own z and y passes
+                           // (r2c / c2r1 unused)
   int div_xc = 0;          // x chunk of the tiled divergence stencil
   // Simulations of the run still active at leapfrog position it (a prefix
   // when the run is ordered by non-increasing step count), and the batched
@@ -376,7 +378,8 @@ void potential_modes(fpm_plan* p, const float2* in, float2* out, float* zero,
     const int n = run_active(r, pos);
     const SimDev& S = p->sims[r.first];
     launch_fft_xpass(p->d_sims, r.first, n, S.mx, S.my, S.mzh, in, out,
-                     zmul == 1 && S.pairs ? nullptr : zero, zmul, tabs_of(p),
+                     zmul == 1 && S.pairs ? nullptr : zero, zmul,
+                     tabs_of(p),
                      G, act, pos, st);
   }
   if (other)
@@ -384,13 +387,18 @@ void potential_modes(fpm_plan* p, const float2* in, float2* out, float* zero,
                              tabs_of(p), G, act, pos, 1, st);
 }
 
-// R2C of the painted density of run r's first n sims into dk (library
-// transforms): z pairs become the plain density in the plan's phi buffer
-// first, which the transform may use as scratch; with zero, the painted
-// density is cleared for the next paint.
+// R2C of the painted density of run r's first n sims into dk; zero: the
+// painted density is cleared for the next paint.  For the library transforms
+// z pairs become the plain density in the plan's phi buffer first, which the
+// transform may use as scratch.
 int density_modes(fpm_plan* p, const Run& r, int n, int zero,
                   const int32_t* act, int pos, cudaStream_t st) {
   const SimDev& S = p->sims[r.first];
+  if (r.zy) {
+    launch_fft_zy_fwd(p->d_sims, r.first, n, S.mx, S.my, S.mz, p->rho, true,
+                      S.pairs, zero && S.pairs, p->dk, act, pos, st);
+    return launch_ok();  // the x pass clears a density that is not in pairs
+  }
   const cufftHandle h = pick(r, n, r.r2c, r.r2c_n);
   if (S.pairs) {
     launch_pair_density(p->d_sims, r.first, n, S.mx, S.my, S.mz,
@@ -407,12 +415,42 @@ int density_modes(fpm_plan* p, const Run& r, int n, int zero,
   return FPM_OK;
 }
 
+// R2C of the plain mesh `in` of run r's first n sims into dk; in may be used
+// as scratch.
+int mesh_modes(fpm_plan* p, const Run& r, int n, float* in, const int32_t* act,
+               int pos, cudaStream_t st) {
+  const SimDev& S = p->sims[r.first];
+  if (r.zy) {
+    launch_fft_zy_fwd(p->d_sims, r.first, n, S.mx, S.my, S.mz, in, false,
+                      false, 0, p->dk, act, pos, st);
+    return launch_ok();
+  }
+  return exec_r2c(pick(r, n, r.r2c, r.r2c_n), in + S.m_off, p->dk + S.s_off,
+                  st);
+}
+
+// C2R of one spectrum per sim (spec, overwritten) of run r's first n sims
+// into the mesh out; with force, runs on the own passes also write the z
+// component of the force.
+int modes_mesh(fpm_plan* p, const Run& r, int n, float2* spec, float* out,
+               bool force, const int32_t* act, int pos, cudaStream_t st) {
+  const SimDev& S = p->sims[r.first];
+  if (r.zy) {
+    launch_fft_zy_inv(p->d_sims, r.first, n, S.mx, S.my, S.mz, spec, out,
+                      force ? p->fmesh : nullptr, act, pos, st);
+    return launch_ok();
+  }
+  return exec_c2r(pick(r, n, r.c2r1, r.c2r1_n), spec + S.s_off, out + S.m_off,
+                  st);
+}
+
 // The three force meshes D_d phi of the sims (with act, those with nsteps
 // >= pos; with skip_fused, not the fused-solve runs, which make their own):
 // the tiled stencil when every run takes the tiled stencils, else the
-// per-chunk one.
+// per-chunk one.  solved: right after the solve, which has left the z
+// component of the runs on its own z pass.
 void stencil_grad(fpm_plan* p, const float* phi, const int32_t* act, int pos,
-                  int skip_fused, cudaStream_t st) {
+                  int skip_fused, cudaStream_t st, bool solved = false) {
   if (!p->div_tiled) {
     launch_stencil_grad(p->d_sims, p->nsims, p->ch_m, phi, p->fmesh, act, pos,
                         skip_fused, p->quads, st);
@@ -424,7 +462,8 @@ void stencil_grad(fpm_plan* p, const float* phi, const int32_t* act, int pos,
     if (n == 0) continue;
     const SimDev& S = p->sims[r.first];
     launch_stencil_grad_tiled(p->d_sims, r.first, n, S.mx, S.my, S.mz,
-                              r.div_xc, phi, p->fmesh, act, pos, st);
+                              r.div_xc, phi, p->fmesh, !(solved && r.zy), act,
+                              pos, st);
   }
 }
 
@@ -501,15 +540,14 @@ int force_meshes(fpm_plan* p, cudaStream_t st, bool zero_rho, int it = -1,
     const int n = run_active(r, it);
     if (n == 0) continue;
     if (stencil_path(p))
-      FPM_TRY(exec_c2r(pick(r, n, r.c2r1, r.c2r1_n), p->fk + S.s_off,
-                       phi + S.m_off, st));
+      FPM_TRY(modes_mesh(p, r, n, p->fk, phi, true, act, it, st));
     else
       FPM_TRY(exec_c2r(pick(r, n, r.c2r3, r.c2r3_n), p->fk + 3 * S.s_off,
                        p->fmesh + 3 * S.m_off, st));
   }
   if (stencil_path(p)) {
     prof_mark(p, 4, st);
-    stencil_grad(p, phi, act, it, 1, st);
+    stencil_grad(p, phi, act, it, 1, st, true);
     prof_mark(p, 4, st);
     FPM_TRY(launch_ok());
   }
@@ -553,13 +591,11 @@ int pgd_meshes(fpm_plan* p, cudaStream_t st, int pos, float* phi = nullptr) {
   FPM_TRY(launch_ok());
   for (auto& r : p->runs) {
     if (r.fused) continue;
-    const SimDev& S = p->sims[r.first];
     const int n = run_active(r, apos);
     if (n == 0) continue;
-    FPM_TRY(exec_c2r(pick(r, n, r.c2r1, r.c2r1_n), p->fk + S.s_off,
-                     phi + S.m_off, st));
+    FPM_TRY(modes_mesh(p, r, n, p->fk, phi, true, act, apos, st));
   }
-  stencil_grad(p, phi, act, apos, 1, st);
+  stencil_grad(p, phi, act, apos, 1, st, true);
   return launch_ok();
 }
 
@@ -821,6 +857,7 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
     if (aligned && fft_xpass_supported(S0.mx, S0.my, S0.mz) &&
         fft_xpass_prepare() == FPM_OK) {
       r.xpass = true;
+      r.zy = fft_zy_supported(S0.my, S0.mz);
       for (int s = r.first; s < r.first + r.count; ++s) p->sims[s].xpass = 1;
     }
   }
@@ -1675,8 +1712,7 @@ static int adjoint_density(fpm_plan* p, int pos, const Green& G,
       continue;
     }
     any_cufft = true;
-    FPM_TRY(exec_r2c(pick(r, n, r.r2c, r.r2c_n), p->phi + S.m_off,
-                     p->dk + S.s_off, st));
+    FPM_TRY(mesh_modes(p, r, n, p->phi, act, pos, st));
   }
   FPM_TRY(launch_ok());
   if (any_cufft) {
@@ -1686,11 +1722,9 @@ static int adjoint_density(fpm_plan* p, int pos, const Green& G,
                     act, pos, st);
     FPM_TRY(launch_ok());
     for (auto& r : p->runs) {
-      const SimDev& S = p->sims[r.first];
       const int n = run_active(r, pos);
       if (n == 0 || r.fused) continue;
-      FPM_TRY(exec_c2r(pick(r, n, r.c2r1, r.c2r1_n), p->dk + S.s_off,
-                       p->lrho + S.m_off, st));
+      FPM_TRY(modes_mesh(p, r, n, p->dk, p->lrho, false, act, pos, st));
     }
   }
   prof_mark(p, 8, st);
