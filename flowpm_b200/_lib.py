@@ -40,6 +40,7 @@ SIGNATURES = {
     'fpm_plan_create': (c_int, [ctypes.POINTER(c_void_p), c_int, P_int32,
                                 c_double, c_uint]),
     'fpm_plan_destroy': (c_int, [c_void_p]),
+    'fpm_plan_set_async': (c_int, [c_void_p, c_int]),
     'fpm_plan_info': (c_int, [c_void_p, P_int64, P_int64]),
     'fpm_plan_status': (c_int, [c_void_p, P_int32, c_void_p]),
     'fpm_force': (c_int, [c_void_p, c_void_p, P_double, c_void_p, c_void_p]),

@@ -23,6 +23,9 @@ class Plan(object):
     _lib.call('fpm_plan_create', ctypes.byref(h), len(self.dims),
               _lib.ivec(flat), self.r_split, self.flags)
     self.handle = h
+    # results are torch tensors, ordered by the stream: a wait after every
+    # table upload only lets the GPU run dry between calls
+    _lib.call('fpm_plan_set_async', h, 1)
     np_tot, nbytes = ctypes.c_int64(), ctypes.c_int64()
     _lib.call('fpm_plan_info', h, ctypes.byref(np_tot), ctypes.byref(nbytes))
     self.total_particles = np_tot.value

@@ -135,6 +135,8 @@ struct fpm_plan {
   void* work = nullptr;
   size_t device_bytes = 0;
   bool steps_set = false;
+  // fpm_plan_set_async: the end of the plan's latest call, or null
+  cudaEvent_t used = nullptr;
   int64_t coef_gen = 0;   // bumped whenever d_coefs is reallocated
   int64_t sched_gen = 0;  // bumped whenever the active-prefix schedule moves
   size_t work_bytes = 0;  // size of the shared cuFFT work area
@@ -225,6 +227,7 @@ void free_all(fpm_plan* p) {
   for (cudaStream_t s : p->side) cudaStreamDestroy(s);
   for (cudaEvent_t e : p->ev_join) cudaEventDestroy(e);
   if (p->ev_fork) cudaEventDestroy(p->ev_fork);
+  if (p->used) cudaEventDestroy(p->used);
   for (int k = 0; k < kProfKinds; ++k)
     for (cudaEvent_t e : p->ev[k]) cudaEventDestroy(e);
   void* bufs[] = {p->d_sims, p->d_kk, p->d_kk2,   p->d_grad,  p->d_win,   p->rho,
@@ -678,6 +681,39 @@ int update_schedule(fpm_plan* p, int max_steps, const int32_t* nsteps,
   return FPM_OK;
 }
 
+// One call on the plan's tables and scratch.  An asynchronous plan's calls do
+// not wait for the stream, so a call on another stream is ordered after the
+// latest one by an event.  A capture takes no events from outside it: a
+// captured call is ordered when its graph is launched.
+class Use {
+ public:
+  Use(const fpm_plan* p, cudaStream_t st) : p_(p), st_(st) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    on_ = p && p->used && cudaStreamIsCapturing(st, &c) == cudaSuccess &&
+          c == cudaStreamCaptureStatusNone;
+    if (on_) cudaStreamWaitEvent(st, p->used, 0);
+  }
+  ~Use() {
+    if (on_) cudaEventRecord(p_->used, st_);
+  }
+  Use(const Use&) = delete;
+  Use& operator=(const Use&) = delete;
+
+ private:
+  const fpm_plan* p_;
+  cudaStream_t st_;
+  bool on_;
+};
+
+// End of a call that uploads host tables: waits for the stream unless the
+// plan is asynchronous.  The wait is part of the call's contract, not needed
+// for the tables themselves: a copy from pageable memory returns when it has
+// been staged.
+int settle(const fpm_plan* p, cudaStream_t st) {
+  if (!p->used) FPM_CUDA(cudaStreamSynchronize(st));
+  return FPM_OK;
+}
+
 // Whether two simulations (nx, ny, nz, bf) share a run.
 bool same_dims(const int32_t* a, const int32_t* b) {
   return a[0] == b[0] && a[1] == b[1] && a[2] == b[2] && a[3] == b[3];
@@ -1005,6 +1041,18 @@ extern "C" int fpm_plan_destroy(fpm_plan* p) {
   return FPM_OK;
 }
 
+extern "C" int fpm_plan_set_async(fpm_plan* p, int enable) {
+  if (!p) return FPM_ERR_ARG;
+  if (enable && !p->used) {
+    FPM_CUDA(cudaEventCreateWithFlags(&p->used, cudaEventDisableTiming));
+  } else if (!enable && p->used) {
+    FPM_CUDA(cudaEventSynchronize(p->used));
+    FPM_CUDA(cudaEventDestroy(p->used));
+    p->used = nullptr;
+  }
+  return FPM_OK;
+}
+
 extern "C" int fpm_plan_info(const fpm_plan* p, int64_t* total_particles,
                              int64_t* device_bytes) {
   if (!p) return FPM_ERR_ARG;
@@ -1014,6 +1062,7 @@ extern "C" int fpm_plan_info(const fpm_plan* p, int64_t* total_particles,
 }
 
 extern "C" int fpm_plan_status(fpm_plan* p, int32_t* status, void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || !status) return FPM_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   int32_t v = 0;
@@ -1027,6 +1076,7 @@ extern "C" int fpm_plan_status(fpm_plan* p, int32_t* status, void* stream) {
 
 extern "C" int fpm_force(fpm_plan* p, const float* disp,
                          const double* force_fac, float* force, void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || !disp || !force_fac || !force) return FPM_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   FPM_TRY(upload_ffac(p, force_fac, st));
@@ -1043,6 +1093,7 @@ extern "C" int fpm_force(fpm_plan* p, const float* disp,
 extern "C" int fpm_nbody_set_steps(fpm_plan* p, int max_steps,
                                    const int32_t* nsteps, const double* coefs,
                                    const double* force_fac, void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || max_steps < 0 || !nsteps || !force_fac ||
       (max_steps > 0 && !coefs))
     return FPM_ERR_ARG;
@@ -1079,8 +1130,7 @@ extern "C" int fpm_nbody_set_steps(fpm_plan* p, int max_steps,
   FPM_CUDA(cudaMemcpyAsync(p->d_nsteps, nsteps, sizeof(int32_t) * p->nsims,
                            cudaMemcpyHostToDevice, st));
   FPM_TRY(upload_ffac(p, force_fac, st));
-  // The uploads read pageable host vectors that die with this call.
-  FPM_CUDA(cudaStreamSynchronize(st));
+  FPM_TRY(settle(p, st));
   FPM_TRY(update_schedule(p, max_steps, nsteps, st));
   p->max_steps = max_steps;
   p->steps_set = true;
@@ -1383,6 +1433,7 @@ int nbody_binned(fpm_plan* p, StepArgs a, cudaStream_t st) {
 extern "C" int fpm_nbody_run(fpm_plan* p, float* disp, float* mom,
                              float* force, float* inter, unsigned flags,
                              float* ckpt, int ckpt_every, void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || !disp || !mom || !force || (ckpt && ckpt_every < 1))
     return FPM_ERR_ARG;
   if (!p->steps_set) return FPM_ERR_STATE;
@@ -1439,6 +1490,7 @@ extern "C" int fpm_nbody_run(fpm_plan* p, float* disp, float* mom,
 
 extern "C" int fpm_nbody_set_pgd(fpm_plan* p, int enable, const double* params,
                                  void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || (enable && !params)) return FPM_ERR_ARG;
   if (!enable) {
     if (p->pgd_on) {
@@ -1475,7 +1527,7 @@ extern "C" int fpm_nbody_set_pgd(fpm_plan* p, int enable, const double* params,
             (float)params[((size_t)s * p->max_steps + t) * 3 + q];
   FPM_CUDA(cudaMemcpyAsync(p->d_pgd, h.data(), sizeof(float) * h.size(),
                            cudaMemcpyHostToDevice, st));
-  FPM_CUDA(cudaStreamSynchronize(st));  // h is pageable and dies here
+  FPM_TRY(settle(p, st));
   if (!p->pgd_on) {
     p->pgd_on = true;
     p->sched_gen++;
@@ -1644,6 +1696,7 @@ extern "C" int fpm_plan_set_adjoint_binning(fpm_plan* p, int sort_every) {
 
 extern "C" int fpm_pgd(fpm_plan* p, float* disp, const double* params,
                        void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || !disp || !params) return FPM_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   if (!p->d_pgd1) {
@@ -1666,14 +1719,14 @@ extern "C" int fpm_pgd(fpm_plan* p, float* disp, const double* params,
   launch_pgd(p->d_sims, p->nsims, traverse_chunks(p), disp, p->fmesh, p->rho,
              p->d_pgd1, 1, 0, nullptr, p->d_status, st);
   FPM_TRY(launch_ok());
-  FPM_CUDA(cudaStreamSynchronize(st));  // h is pageable and dies here
-  return FPM_OK;
+  return settle(p, st);
 }
 
 extern "C" int fpm_nbody(fpm_plan* p, float* disp, float* mom, float* force,
                          int max_steps, const int32_t* nsteps,
                          const double* coefs, const double* force_fac,
                          float* inter, unsigned flags, void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   FPM_TRY(fpm_nbody_set_steps(p, max_steps, nsteps, coefs, force_fac, stream));
   return fpm_nbody_run(p, disp, mom, force, inter, flags, nullptr, 0, stream);
 }
@@ -1885,6 +1938,7 @@ extern "C" int fpm_nbody_adjoint(fpm_plan* p, float* disp, float* mom,
                                  float* lam_p, const float* lam_f,
                                  const float* ckpt, int ckpt_every,
                                  void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || !disp || !mom || !force || !lam_x || !lam_p ||
       (ckpt && ckpt_every < 1))
     return FPM_ERR_ARG;
@@ -1954,6 +2008,7 @@ extern "C" int fpm_nbody_set_tape(fpm_plan* p, float* tape, int64_t floats) {
 extern "C" int fpm_lpt_init(fpm_plan* p, const float* linear,
                             const double* coef, int order, float* disp,
                             float* mom, float* force, void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || !linear || !coef || !disp || !mom || !force ||
       (order != 1 && order != 2))
     return FPM_ERR_ARG;
@@ -1999,13 +2054,12 @@ extern "C" int fpm_lpt_init(fpm_plan* p, const float* linear,
   launch_lpt_particles(p->d_sims, p->nsims, p->ch_p, p->lreal9, 9, psi2, 3,
                        p->d_lcoef, disp, mom, force, st);
   FPM_TRY(launch_ok());
-  // The coefficient upload reads a host vector that dies with this call.
-  FPM_CUDA(cudaStreamSynchronize(st));
-  return FPM_OK;
+  return settle(p, st);
 }
 
 extern "C" int fpm_lpt1(fpm_plan* p, const void* dlin_kv, const float* pos,
                         int64_t npart, float* disp, void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   const float2* dlin_k = (const float2*)dlin_kv;
   if (!p || !dlin_k || !pos || !disp || npart < 0) return FPM_ERR_ARG;
   if (!(p->flags & FPM_PLAN_LPT)) return FPM_ERR_STATE;
@@ -2027,6 +2081,7 @@ extern "C" int fpm_lpt1(fpm_plan* p, const void* dlin_kv, const float* pos,
 
 extern "C" int fpm_lpt2_source(fpm_plan* p, const void* dlin_kv,
                                void* source_kv, void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   const float2* dlin_k = (const float2*)dlin_kv;
   float2* source_k = (float2*)source_kv;
   if (!p || !dlin_k || !source_k) return FPM_ERR_ARG;
@@ -2058,6 +2113,7 @@ extern "C" int fpm_lpt_adjoint(fpm_plan* p, const float* linear,
                                const float* lam_disp, const float* lam_mom,
                                const float* lam_force, float* lam_linear,
                                void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || !linear || !coef || !lam_disp || !lam_linear ||
       (order != 1 && order != 2))
     return FPM_ERR_ARG;
@@ -2120,13 +2176,13 @@ extern "C" int fpm_lpt_adjoint(fpm_plan* p, const float* linear,
     const SimDev& S = p->sims[r.first];
     FPM_TRY(exec_c2r(r.lc2r1, p->lspec1 + S.ls_off, lam_linear + S.l_off, st));
   }
-  FPM_CUDA(cudaStreamSynchronize(st));
-  return FPM_OK;
+  return settle(p, st);
 }
 
 extern "C" int fpm_linear_field(fpm_plan* p, const float* amp, uint64_t seed,
                                 int generate, float* white, float* linear,
                                 void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || !amp || !linear || (!generate && !white)) return FPM_ERR_ARG;
   if (!(p->flags & FPM_PLAN_LPT)) return FPM_ERR_STATE;
   cudaStream_t st = (cudaStream_t)stream;
@@ -2277,6 +2333,7 @@ extern "C" int fpm_graph_launch(fpm_graph* g, void* stream) {
   if (g->plan->max_steps != g->max_steps ||
       g->plan->coef_gen != g->coef_gen || g->plan->sched_gen != g->sched_gen)
     return FPM_ERR_STATE;
+  const Use use(g->plan, (cudaStream_t)stream);
   FPM_CUDA(cudaGraphLaunch(g->exec, (cudaStream_t)stream));
   return FPM_OK;
 }
@@ -2456,6 +2513,7 @@ std::vector<int64_t> tune_key(const fpm_plan* p) {
 extern "C" int fpm_plan_autotune(fpm_plan* p, const float* disp,
                                  const float* mom, int reps, int retune,
                                  int32_t* choice, float* ms, void* stream) {
+  const Use use(p, (cudaStream_t)stream);
   if (!p || !choice || reps < 1 || (!retune && !disp) != (!retune && !mom) ||
       (retune && (!disp || !mom)))
     return FPM_ERR_ARG;

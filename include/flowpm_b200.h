@@ -156,6 +156,13 @@ int fpm_plan_destroy(fpm_plan* plan);
 /* Total particles of the plan and bytes of device memory it holds. */
 int fpm_plan_info(const fpm_plan* plan, int64_t* total_particles,
                   int64_t* device_bytes);
+/* With enable, the plan's calls that are noted to synchronise the stream
+ * (fpm_nbody_set_steps, fpm_nbody_set_pgd, fpm_pgd, fpm_lpt_init,
+ * fpm_lpt_adjoint) are stream-ordered only, and the plan's calls and graph
+ * launches on different streams run one after the other; fpm_plan_status
+ * still synchronises.  Off for a new plan. */
+int fpm_plan_set_async(fpm_plan* plan, int enable);
+
 /* Copy the device status word to *status and clear it (synchronises the
  * stream). */
 int fpm_plan_status(fpm_plan* plan, int32_t* status, void* stream);
