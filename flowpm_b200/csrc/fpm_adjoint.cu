@@ -594,65 +594,6 @@ k_adj_fourier(const SimDev* __restrict__ sims, int nsims, int64_t nchunks,
 }
 
 // ---------------------------------------------------------------------------
-// Stand-alone CIC adjoints (uniform batch)
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads)
-k_cic_paint_adjoint(const float* __restrict__ lmesh, int nx, int ny, int nz,
-                    const float* __restrict__ part, int64_t npart,
-                    int64_t total, const float* __restrict__ weight,
-                    float* __restrict__ lpart, float* __restrict__ lweight) {
-  const int64_t ncell = (int64_t)nx * ny * nz;
-  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total;
-       g += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = g / npart;
-    const float3 y = ld3(part, g);
-    const float* m = lmesh + b * ncell;
-    const float wt = weight ? weight[g] : 1.f;
-    if (lpart) {
-      const float3 gg = gather_grad(m, nx, ny, nz, y);
-      st3(lpart, g, make_float3(wt * gg.x, wt * gg.y, wt * gg.z));
-    }
-    if (lweight) {
-      const Axis ax = cic_axis(y.x, nx), ay = cic_axis(y.y, ny),
-                 az = cic_axis(y.z, nz);
-      float acc = 0.f;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const int cx = conn_x(c), cy = conn_y(c), cz = conn_z(c);
-        const int ix = cx ? ax.i1 : ax.i0, iy = cy ? ay.i1 : ay.i0,
-                  iz = cz ? az.i1 : az.i0;
-        acc += __ldg(m + ((int64_t)ix * ny + iy) * nz + iz) *
-               cic_w(ax, ay, az, cx, cy, cz);
-      }
-      lweight[g] = acc;
-    }
-  }
-}
-
-__global__ void __launch_bounds__(kThreads)
-k_cic_readout_adjoint(const float* __restrict__ mesh, int nx, int ny, int nz,
-                      const float* __restrict__ part, int64_t npart,
-                      int64_t total, const float* __restrict__ lout,
-                      float* __restrict__ lmesh, float* __restrict__ lpart) {
-  const int64_t ncell = (int64_t)nx * ny * nz;
-  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total;
-       g += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = g / npart;
-    const float3 y = ld3(part, g);
-    const float lo = lout[g];
-    if (lpart) {
-      const float3 gg = gather_grad(mesh + b * ncell, nx, ny, nz, y);
-      st3(lpart, g, make_float3(lo * gg.x, lo * gg.y, lo * gg.z));
-    }
-    if (lmesh) {
-      const Axis ax = cic_axis(y.x, nx), ay = cic_axis(y.y, ny),
-                 az = cic_axis(y.z, nz);
-      paint_scaled(lmesh + b * ncell, nx, ny, nz, ax, ay, az, lo);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
 // LPT adjoint (flowpm/tfpm.py:148-180 lpt_init, :66-145 lpt1 / lpt2_source)
 // ---------------------------------------------------------------------------
 
@@ -846,49 +787,3 @@ void launch_lpt_adj_phi(const SimDev* sims, int nsims, int64_t nchunks,
 }
 
 }  // namespace fpm
-
-using namespace fpm;
-
-static unsigned grid_elems_adj(int64_t n) {
-  int64_t blocks = (n + kThreads - 1) / kThreads;
-  const int64_t cap = (int64_t)kNumSMs * 32;
-  if (blocks < 1) blocks = 1;
-  return (unsigned)(blocks < cap ? blocks : cap);
-}
-
-extern "C" int fpm_cic_paint_adjoint(const float* lam_mesh, int batch, int nx,
-                                     int ny, int nz, const float* part,
-                                     int64_t npart, const float* weight,
-                                     float* lam_part, float* lam_weight,
-                                     void* stream) {
-  if (!lam_mesh || batch < 1 || nx < 1 || ny < 1 || nz < 1 || npart < 0 ||
-      (npart > 0 && !part) || (!lam_part && !lam_weight))
-    return FPM_ERR_ARG;
-  const int64_t total = (int64_t)batch * npart;
-  if (total == 0) return FPM_OK;
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_cic_paint_adjoint<<<grid_elems_adj(total), kThreads, 0,
-                        (cudaStream_t)stream>>>(lam_mesh, nx, ny, nz, part,
-                                                npart, total, weight, lam_part,
-                                                lam_weight);
-  return cudaGetLastError() == cudaSuccess ? FPM_OK : FPM_ERR_CUDA;
-}
-
-extern "C" int fpm_cic_readout_adjoint(const float* mesh, int batch, int nx,
-                                       int ny, int nz, const float* part,
-                                       int64_t npart, const float* lam_out,
-                                       float* lam_mesh, float* lam_part,
-                                       void* stream) {
-  if (batch < 1 || nx < 1 || ny < 1 || nz < 1 || npart < 0 ||
-      (npart > 0 && (!part || !lam_out)) || (!lam_mesh && !lam_part) ||
-      (lam_part && !mesh))
-    return FPM_ERR_ARG;
-  const int64_t total = (int64_t)batch * npart;
-  if (total == 0) return FPM_OK;
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_cic_readout_adjoint<<<grid_elems_adj(total), kThreads, 0,
-                          (cudaStream_t)stream>>>(mesh, nx, ny, nz, part,
-                                                  npart, total, lam_out,
-                                                  lam_mesh, lam_part);
-  return cudaGetLastError() == cudaSuccess ? FPM_OK : FPM_ERR_CUDA;
-}

@@ -530,21 +530,6 @@ __device__ __forceinline__ Cic8 cic8(const Axis& ax, const Axis& ay,
   return c;
 }
 
-// Deposit s * W at the 8 neighbours (s = 1: plain paint).
-__device__ __forceinline__ void paint_cic8(float* __restrict__ m,
-                                           const Cic8& c, float s) {
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    float w0 = __fmul_rn(c.wxy[q], c.wz0), w1 = __fmul_rn(c.wxy[q], c.wz1);
-    if (s != 1.f) {
-      w0 = __fmul_rn(s, w0);
-      w1 = __fmul_rn(s, w1);
-    }
-    red_add(m + c.row[q] + c.z0, w0);
-    red_add(m + c.row[q] + c.z1, w1);
-  }
-}
-
 // Deposit of the step kernels into a simulation's painted density m; w[2 q],
 // w[2 q + 1]: the weights of row q.
 //
@@ -599,14 +584,6 @@ __device__ __forceinline__ Cic8 cic8_at(const SimDev& S, float3 x) {
   Axis ax, ay, az;
   cic_axes(x, S.mx, S.my, S.mz, ax, ay, az);
   return cic8(ax, ay, az, S.my, S.mz);
-}
-
-// Deposit s * W at the 8 neighbours.
-__device__ __forceinline__ void paint_scaled(float* __restrict__ m, int mx,
-                                             int my, int mz, const Axis& ax,
-                                             const Axis& ay, const Axis& az,
-                                             float s) {
-  paint_cic8(m, cic8(ax, ay, az, my, mz), s);
 }
 
 // Readout of the three force components (planes f0, f0 + mcells,
