@@ -78,26 +78,28 @@ class CicPaint2D(torch.autograd.Function):
 
 
 class DensityPlanes(torch.autograd.Function):
-  """Planes of positions X (batch, npart, 3); ``args`` = the host
-  parameters of fpm_density_planes after X."""
+  """Planes of the positions state[0] (batch, npart, 3); ``args`` = the host
+  parameters of fpm_density_planes after X.  The cotangent of the whole state
+  is written in place: the positions' by the library, zeros for the rest."""
 
   @staticmethod
-  def forward(ctx, X, args):
-    out = torch.empty(args['shape'], dtype=torch.float32, device=X.device)
-    _lib.call('fpm_density_planes', _lib.ptr(X.detach()), *args['c'],
-              _lib.ptr(out), _lib.stream_ptr())
-    ctx.save_for_backward(X)
+  def forward(ctx, state, args):
+    out = torch.empty(args['shape'], dtype=torch.float32, device=state.device)
+    _lib.call('fpm_density_planes_async', _lib.ptr(state.detach()),
+              *args['c'], _lib.ptr(out), _lib.stream_ptr())
+    ctx.save_for_backward(state)
     ctx.args = args
     return out
 
   @staticmethod
   def backward(ctx, g):
-    (X,) = ctx.saved_tensors
-    gX = torch.empty_like(X)
-    _lib.call('fpm_density_planes_adjoint', _lib.ptr(X.detach()),
-              *ctx.args['c'], _lib.ptr(g.contiguous()), _lib.ptr(gX),
+    (state,) = ctx.saved_tensors
+    gs = torch.empty_like(state)
+    gs[1:].zero_()
+    _lib.call('fpm_density_planes_adjoint', _lib.ptr(state.detach()),
+              *ctx.args['c'], _lib.ptr(g.contiguous()), _lib.ptr(gs),
               _lib.stream_ptr())
-    return gX, None
+    return gs, None
 
 
 class CicReadout(torch.autograd.Function):

@@ -122,6 +122,10 @@ SIGNATURES = {
                                    c_int, P_double, P_double, c_int,
                                    P_double, P_double, c_int, c_void_p,
                                    c_void_p]),
+    'fpm_density_planes_async': (c_int, [c_void_p, c_int, c_int64, c_int,
+                                         c_int, c_int, P_double, P_double,
+                                         c_int, P_double, P_double, c_int,
+                                         c_void_p, c_void_p]),
     'fpm_density_planes_adjoint': (c_int, [c_void_p, c_int, c_int64, c_int,
                                            c_int, c_int, P_double, P_double,
                                            c_int, P_double, P_double, c_int,

@@ -21,8 +21,8 @@ def _nc3(nc):
   return [nc] * 3 if isinstance(nc, int) else [int(n) for n in nc]
 
 
-def _planes(X, nc, centers, widths, res, rotation, shift):
-  B, npart = X.shape[0], X.shape[1]
+def _planes(state, nc, centers, widths, res, rotation, shift):
+  B, npart = state.shape[1], state.shape[2]
   nx, ny, nz = nc
   rot = None if rotation is None else _lib.dvec(
       np.asarray(rotation, dtype=np.float64).reshape(9))
@@ -33,11 +33,11 @@ def _planes(X, nc, centers, widths, res, rotation, shift):
       'c': (B, npart, nx, ny, nz, rot, sh, len(centers), _lib.dvec(centers),
             _lib.dvec(widths), res),
   }
-  if _autograd.needs_grad(X):
-    return _autograd.DensityPlanes.apply(X, args)
-  out = torch.empty(args['shape'], dtype=torch.float32, device=X.device)
-  _lib.call('fpm_density_planes', _lib.ptr(X), *args['c'], _lib.ptr(out),
-            _lib.stream_ptr())
+  if _autograd.needs_grad(state):
+    return _autograd.DensityPlanes.apply(state, args)
+  out = torch.empty(args['shape'], dtype=torch.float32, device=state.device)
+  _lib.call('fpm_density_planes_async', _lib.ptr(state), *args['c'],
+            _lib.ptr(out), _lib.stream_ptr())
   return out
 
 
@@ -49,14 +49,16 @@ def density_planes(state, nc, centers, widths, plane_resolution,
   (fractions of the box): the transform, the 2-D periodic wrap and the
   normalisation of flowpm/raytracing.py:49-109."""
   nc = _nc3(nc)
-  X = as_cuda(state)[0]
+  state = as_cuda(state)
   centers = [float(c) for c in np.atleast_1d(centers)]
   widths = np.broadcast_to(np.asarray(widths, dtype=np.float64),
                            (len(centers),)).tolist()
   res = int(plane_resolution)
+  if len(centers) > MAX_PLANES:
+    state = state[:1]  # the parts' cotangents are summed: positions only
   parts = []
   for i in range(0, len(centers), MAX_PLANES):
-    parts.append(_planes(X, nc, centers[i:i + MAX_PLANES],
+    parts.append(_planes(state, nc, centers[i:i + MAX_PLANES],
                          widths[i:i + MAX_PLANES], res, rotation, shift))
   return parts[0] if len(parts) == 1 else torch.cat(parts, dim=1)
 

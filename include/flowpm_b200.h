@@ -557,12 +557,18 @@ int fpm_cic_paint_2d_adjoint(const float* grad_mesh, int batch, int nx,
  * nx, ny, nz), each NULL for none; xy modulo nx, scaled by res / nx;
  * particles with center - width/2 < z <= center + width/2 painted into
  * slab p of planes (batch, nplanes, res, res), which is then divided by
- * (nx / res) (ny / res) width.  Synchronises the stream. */
+ * (nx / res) (ny / res) width.  Synchronises the stream;
+ * fpm_density_planes_async does not. */
 int fpm_density_planes(const float* X, int batch, int64_t npart, int nx,
                        int ny, int nz, const double* rotation,
                        const double* shift, int nplanes, const double* centers,
                        const double* widths, int res, float* planes,
                        void* stream);
+int fpm_density_planes_async(const float* X, int batch, int64_t npart, int nx,
+                             int ny, int nz, const double* rotation,
+                             const double* shift, int nplanes,
+                             const double* centers, const double* widths,
+                             int res, float* planes, void* stream);
 /* Its adjoint: grad_X (batch, npart, 3) for the plane cotangent. */
 int fpm_density_planes_adjoint(const float* X, int batch, int64_t npart,
                                int nx, int ny, int nz, const double* rotation,
