@@ -140,11 +140,9 @@ class LptInit(torch.autograd.Function):
                         device=linear.device)
     st = _lib.stream_ptr()
     lin = linear.detach().contiguous()
-    _lib.call('fpm_lpt_init', plan.handle, _lib.ptr(lin), _lib.dvec(coef),
+    _lib.call('fpm_lpt_state', plan.handle, _lib.ptr(lin), _lib.dvec(coef),
               order, _lib.ptr(state[0]), _lib.ptr(state[1]),
               _lib.ptr(state[2]), st)
-    _lib.call('fpm_lattice_shift', _lib.ptr(state[0]), _lib.ptr(state[0]), B,
-              nx, ny, nz, 1, st)
     ctx.save_for_backward(lin)
     ctx.coef, ctx.order = coef, order
     return state

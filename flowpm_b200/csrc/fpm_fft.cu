@@ -804,6 +804,398 @@ k_fft_y(const SimDev* __restrict__ sims, int first, float2* __restrict__ dk,
   }
 }
 
+// ---------------------------------------------------------------------------
+// 2LPT on the particle lattice (flowpm/tfpm.py:148-180 lpt_init) for
+// power-of-two axes of 16 to 512.  A displacement or a second derivative of
+// the potential is the Laplacian's inverse T times a factor per axis and a
+// power of i, so the factor of an axis is applied where that axis is
+// transformed back and the outputs share the passes before it:
+//
+//   rows forward, k_lpt_y_fwd     linear field -> spectrum along (y, z)
+//   k_lpt_x       forward and back along x of T, gx T, gx^2 T
+//   k_lpt_y_inv   back along y of gy^b (gx^a T), a + b <= 2: six spectra
+//   k_lpt_rows_source  back along z of the six second derivatives of a row,
+//                 the second-order source, and its row forward again
+//   k_lpt_y_fwd, k_lpt_x, k_lpt_y_inv  of the source: three spectra
+//   k_lpt_rows_out  back along z of both displacements; disp, mom and force
+//
+// Bound by memory: 49 passes over a field of 4 bytes per cell, against 98 of
+// one transform per output (library transforms of three passes each, a
+// kernel for the spectra, the source and the particles).  Measured on B200,
+// 256^3 to second order with positions: 1.82 -> 0.85 ms (3.3 GB, 3.9 TB/s;
+// y back 117 us a pass, rows out 229, source 156, x 66).
+// ---------------------------------------------------------------------------
+
+// Spectrum row <-> the lane's elements k = g + N2 u + N1 k2, X[0] and X[M]
+// (both real) in one.
+template <int M>
+__device__ __forceinline__ int row_k(int g, int e) {
+  constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2;
+  return g + N2 * (e / N2) + N1 * (e % N2);
+}
+
+template <int M>
+__device__ __forceinline__ void spec_put(const float2 (&a)[Split<M>::N1],
+                                         float2* o, int g) {
+#pragma unroll
+  for (int e = 0; e < Split<M>::N1; ++e) {
+    float2 v = a[e];
+    if (e == 0 && g == 0) {
+      o[M] = make_float2(v.y, 0.f);
+      v.y = 0.f;
+    }
+    o[row_k<M>(g, e)] = v;
+  }
+}
+
+// The row x as stored; mid: X[M] (lane g = 0).
+template <int M>
+__device__ __forceinline__ void spec_get(float2 (&a)[Split<M>::N1],
+                                         float2& mid, const float2* x, int g) {
+#pragma unroll
+  for (int e = 0; e < Split<M>::N1; ++e) a[e] = x[row_k<M>(g, e)];
+  mid = g ? make_float2(0.f, 0.f) : x[M];
+}
+
+// Times gz^p and, with I, times i; then packed for row_c2r.
+template <int M, bool I>
+__device__ __forceinline__ void spec_factor(float2 (&a)[Split<M>::N1],
+                                            float2 mid, const float* gz, int p,
+                                            int g) {
+  if (p > 0) {
+    const float gm = __ldg(gz + M);
+#pragma unroll
+    for (int e = 0; e < Split<M>::N1; ++e) {
+      const float f = __ldg(gz + row_k<M>(g, e));
+      a[e].x *= f;
+      a[e].y *= f;
+      if (p > 1) {
+        a[e].x *= f;
+        a[e].y *= f;
+      }
+    }
+    mid.x *= gm;
+    mid.y *= gm;
+    if (p > 1) {
+      mid.x *= gm;
+      mid.y *= gm;
+    }
+  }
+  if (I) {
+#pragma unroll
+    for (int e = 0; e < Split<M>::N1; ++e) a[e] = make_float2(-a[e].y, a[e].x);
+    mid.x = -mid.y;
+  }
+  if (g == 0) a[0].y = mid.x;
+}
+
+// Pitch of the rows of M + 1 modes: whole sectors, so that 16 consecutive
+// columns are four of them.  The columns of the padding are transformed too
+// (nothing reads them).  A pitch of whole lines (M + 16) was no faster.
+template <int M>
+__host__ __device__ constexpr int lpt_pitch() {
+  return M + 4;
+}
+
+constexpr int kLptZThreads = 128;  // row kernels of one row at a time
+constexpr int kLptOutThreads = 96;
+
+// nrows (all simulations of the run) is a multiple of the rows of a warp.
+template <int M>
+__global__ void __launch_bounds__(kLptZThreads, 4)
+k_lpt_rows_fwd(const float* __restrict__ in, float2* __restrict__ out,
+               int nrows) {
+  constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2, RW = 32 / N2;
+  __shared__ float2 ex_[kLptZThreads / N2][M + 8];
+  const int lane = threadIdx.x & 31, g = lane % N2, wpb = kLptZThreads / 32;
+  RowTw<M> tw;
+  tw.load(g);
+  for (int r0 = (blockIdx.x * wpb + (threadIdx.x >> 5)) * RW; r0 < nrows;
+       r0 += gridDim.x * wpb * RW) {
+    const int r = r0 + lane / N2;
+    const float2* p = reinterpret_cast<const float2*>(in) + (size_t)r * M;
+    float2 a[N1];
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) a[j1] = p[N2 * j1 + g];
+    row_r2c<M>(a, ex_[threadIdx.x / N2], g, lane, tw);
+    spec_put<M>(a, out + (size_t)r * lpt_pitch<M>(), g);
+  }
+}
+
+// Forward along y, in place; columns (x, kz) of all simulations of the run.
+template <int NY>
+__global__ void __launch_bounds__(x_threads<NY>(), x_blocks<NY>())
+k_lpt_y_fwd(float2* __restrict__ dk, unsigned nzh) {
+  constexpr int N1 = Split<NY>::N1, N2 = Split<NY>::N2, C = kXCols;
+  extern __shared__ __align__(16) float2 smem[];
+  const int cl = threadIdx.x % C, g = threadIdx.x / C;
+  const unsigned q = blockIdx.x * C + cl;  // nx is a multiple of 16
+  const unsigned x = q / nzh, kz = q - x * nzh;
+  float2* col = dk + (size_t)x * NY * nzh + kz;
+  float2* ex = smem + cl;
+  float2 a[N1];
+#pragma unroll
+  for (int j1 = 0; j1 < N1; ++j1) a[j1] = col[(N2 * j1 + g) * nzh];
+  col_fwd_put<NY>(a, ex, C, g);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < N1 / N2; ++u) {
+    float2 b[N2];
+    col_fwd_get<NY>(b, ex, C, g, u);
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) col[(g + N2 * u + N1 * k2) * nzh] = b[k2];
+  }
+}
+
+// Blocks of the kernels below that the registers of an SM should hold (at 256
+// unbounded, one: the y pass back 166 against 126 us; three spill and gain
+// nothing).
+template <int N>
+__host__ __device__ constexpr int lpt_blocks() {
+  return N == 512 ? 1 : N == 256 ? 2 : N == 128 ? 4 : 8;
+}
+
+// Column v (in kx or ky order of the transform) back along its axis, n times:
+// as it is, then times the axis factor each.  Output d goes to o + slot[d].
+template <int N>
+__device__ __forceinline__ void lpt_outputs(float2 (&v)[Split<N>::N1],
+                                            float2* ex, int g, int n,
+                                            const float* gr, float2* o,
+                                            size_t stride, longlong3 slot) {
+  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2, C = kXCols;
+#pragma unroll 1
+  for (int d = 0; d < n; ++d) {
+    if (d > 0) {
+#pragma unroll
+      for (int e = 0; e < N1; ++e) {
+        const float f = __ldg(gr + g + N2 * (e / N2) + N1 * (e % N2));
+        v[e].x *= f;
+        v[e].y *= f;
+      }
+    }
+    __syncthreads();  // the exchange is free
+#pragma unroll
+    for (int u = 0; u < N1 / N2; ++u) {
+      float2 b[N2];
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) b[k2] = v[u * N2 + k2];
+      col_inv_put<N>(b, ex, C, g, u);
+    }
+    __syncthreads();
+    float2 f[N1];
+    col_inv_get<N>(f, ex, C, g);
+    float2* w = o + (d == 0 ? slot.x : d == 1 ? slot.y : slot.z);
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) w[(N2 * j1 + g) * stride] = f[j1];
+  }
+}
+
+// Forward along x, the inverse Laplacian, back along x: nout of T, gx T and
+// gx^2 T.  kk2, gx: the lattice's axis tables.
+template <int NX>
+__global__ void __launch_bounds__(x_threads<NX>(), lpt_blocks<NX>())
+k_lpt_x(const float2* __restrict__ in, float2* __restrict__ out,
+        int64_t slot, int nblk, unsigned ny, unsigned nzh,
+        const float2* __restrict__ kk2, const float* __restrict__ gx,
+        int nout) {
+  constexpr int N1 = Split<NX>::N1, N2 = Split<NX>::N2, C = kXCols;
+  extern __shared__ __align__(16) float2 smem[];
+  const unsigned ncols = ny * nzh;
+  const int cl = threadIdx.x % C, g = threadIdx.x / C;
+  const int b0 = blockIdx.x / nblk;
+  const unsigned c = (blockIdx.x - b0 * nblk) * C + cl;  // ny % 16 == 0
+  const size_t at = (size_t)b0 * NX * ncols + c;
+  float2* ex = smem + cl;
+  const float2* src = in + at + (size_t)g * ncols;
+  float2 v[N1];
+#pragma unroll
+  for (int j1 = 0; j1 < N1; ++j1) v[j1] = src[(size_t)(N2 * j1) * ncols];
+  const unsigned ky = c / nzh, kz = c - ky * nzh;
+  const unsigned nz = 2 * (nzh - 4);
+  const float pre = (float)(1.0 / ((double)NX * ny * nz));
+  const float2 kyz = two_add(kk2[NX + ky], kk2[NX + ny + min(kz, nz / 2)]);
+  col_fwd_put<NX>(v, ex, C, g);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < N1 / N2; ++u) {
+    float2 b[N2];
+    col_fwd_get<NX>(b, ex, C, g, u);
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) {
+      // 0 at k = 0, where the reference's 1 meets a gradient of 0
+      const float w = green_inv(kk2[g + N2 * u + N1 * k2], kyz);
+      v[u * N2 + k2] = make_float2(__fmul_rn(__fmul_rn(b[k2].x, pre), w),
+                                   __fmul_rn(__fmul_rn(b[k2].y, pre), w));
+    }
+  }
+  lpt_outputs<NX>(v, ex, g, nout, gx, out + at, ncols,
+                  longlong3{0, slot, 2 * slot});
+}
+
+// Back along y of gy^b t[a], b <= nout - 1 - a for the nout spectra t of
+// k_lpt_x, into the slots o[] in the order (a, b) = (0, 0), (0, 1), ...
+struct LptSlots {
+  int o[6];
+};
+template <int NY>
+__global__ void __launch_bounds__(x_threads<NY>(), lpt_blocks<NY>())
+k_lpt_y_inv(const float2* __restrict__ t, float2* __restrict__ u,
+            int64_t slot, unsigned nzh, const float* __restrict__ gy, int nout,
+            const __grid_constant__ LptSlots S) {
+  constexpr int N1 = Split<NY>::N1, N2 = Split<NY>::N2, C = kXCols;
+  extern __shared__ __align__(16) float2 smem[];
+  const int cl = threadIdx.x % C, g = threadIdx.x / C;
+  const unsigned q = blockIdx.x * C + cl;
+  const unsigned x = q / nzh, kz = q - x * nzh;
+  const size_t at = (size_t)x * NY * nzh + kz;
+  int k = 0;
+#pragma unroll 1
+  for (int a = 0; a < nout; ++a) {
+    const float2* col = t + a * slot + at;
+    float2 v[N1];
+#pragma unroll
+    for (int e = 0; e < N1; ++e)
+      v[e] = col[(size_t)(g + N2 * (e / N2) + N1 * (e % N2)) * nzh];
+    const int n = nout - a;
+    lpt_outputs<NY>(v, smem + cl, g, n, gy, u + at, nzh,
+                    longlong3{S.o[k] * slot, n > 1 ? S.o[k + 1] * slot : 0,
+                              n > 2 ? S.o[k + 2] * slot : 0});
+    k += n;
+  }
+}
+
+// Rows of the six spectra u -> second derivatives (their common sign dropped,
+// as the source is quadratic) -> source, forward along z.
+template <int M>
+__global__ void __launch_bounds__(kLptZThreads, 3)
+k_lpt_rows_source(const float2* __restrict__ u, int64_t slot,
+                  float2* __restrict__ out, int nrows,
+                  const float* __restrict__ gz) {
+  constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2, RW = 32 / N2;
+  __shared__ float2 ex_[kLptZThreads / N2][M + 8];
+  const int lane = threadIdx.x & 31, g = lane % N2, wpb = kLptZThreads / 32;
+  float2* ex = ex_[threadIdx.x / N2];
+  RowTw<M> tw;
+  tw.load(g);
+  const float c37 = (float)(3.0 / 7.0);
+  for (int r0 = (blockIdx.x * wpb + (threadIdx.x >> 5)) * RW; r0 < nrows;
+       r0 += gridDim.x * wpb * RW) {
+    const size_t at = (size_t)(r0 + lane / N2) * lpt_pitch<M>();
+    float2 s[N1], t[N1];
+#pragma unroll 1
+    for (int d = 0; d < 6; ++d) {
+      // xx, yy, zz, yz, zx, xy = slots 5, 2, 0, 1, 3, 4 times gz^p
+      const int from = d == 0 ? 5 : d == 1 ? 2 : d == 2 ? 0 : d == 3 ? 1
+                                                      : d == 4 ? 3 : 4;
+      const int p = d == 2 ? 2 : d == 3 || d == 4 ? 1 : 0;
+      float2 a[N1], mid;
+      spec_get<M>(a, mid, u + from * slot + at, g);
+      spec_factor<M, false>(a, mid, gz, p, g);
+      row_c2r<M>(a, ex, g, lane, tw);
+#pragma unroll
+      for (int j = 0; j < N1; ++j) {
+        if (d == 0) {
+          s[j] = a[j];
+        } else if (d == 1) {
+          t[j] = make_float2(__fadd_rn(s[j].x, a[j].x),
+                             __fadd_rn(s[j].y, a[j].y));
+          s[j] = make_float2(__fmul_rn(s[j].x, a[j].x),
+                             __fmul_rn(s[j].y, a[j].y));
+        } else if (d == 2) {
+          s[j].x = __fmaf_rn(t[j].x, a[j].x, s[j].x);
+          s[j].y = __fmaf_rn(t[j].y, a[j].y, s[j].y);
+        } else {
+          s[j].x = __fmaf_rn(-a[j].x, a[j].x, s[j].x);
+          s[j].y = __fmaf_rn(-a[j].y, a[j].y, s[j].y);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < N1; ++j)
+      s[j] = make_float2(__fmul_rn(s[j].x, c37), __fmul_rn(s[j].y, c37));
+    row_r2c<M>(s, ex, g, lane, tw);
+    spec_put<M>(s, out + at, g);
+  }
+}
+
+// Rows of the displacement spectra -> disp (positions with shift), mom and
+// force of the row's particles.  Warp d of a block takes component d of the
+// same rows, the first-order displacement from slot 3, 1 or 0 and the second
+// (order 2) from 5, 4 or 2, both in registers; the arrays, interleaved x, y, z,
+// go through shared memory one after the other, through two buffers in turn.
+template <int M>
+__global__ void __launch_bounds__(kLptOutThreads, 4)
+k_lpt_rows_out(const float2* __restrict__ u, int64_t slot, int order,
+               const float* __restrict__ gz, const float* __restrict__ coef,
+               int nrows, unsigned nx, unsigned ny, int shift,
+               float* __restrict__ disp, float* __restrict__ mom,
+               float* __restrict__ force) {
+  constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2, RW = 32 / N2;
+  constexpr int NZ = 2 * M, P = 3 * NZ + 16;  // rows on different banks
+  __shared__ float2 ex_[kLptOutThreads / N2][M + 8];
+  __shared__ __align__(16) float stage[2][RW * P];
+  const int lane = threadIdx.x & 31, g = lane % N2, d = threadIdx.x >> 5;
+  float2* ex = ex_[threadIdx.x / N2];
+  RowTw<M> tw;
+  tw.load(g);
+  int buf = 0;
+  for (int r0 = blockIdx.x * RW; r0 < nrows; r0 += gridDim.x * RW) {
+    const unsigned r = r0 + lane / N2;
+    const size_t at = (size_t)r * lpt_pitch<M>();
+    const unsigned x = r / ny, b = x / nx;  // one b for the rows of a block
+    const float* c = coef + 6 * b;
+    float2 p1[N1], p2[N1], mid;
+    spec_get<M>(p1, mid, u + (d == 0 ? 3 : d == 1 ? 1 : 0) * slot + at, g);
+    spec_factor<M, true>(p1, mid, gz, d == 2, g);
+    row_c2r<M>(p1, ex, g, lane, tw);
+    const float c0 = c[0], c1 = c[1];
+    if (order == 2) {
+      spec_get<M>(p2, mid, u + (d == 0 ? 5 : d == 1 ? 4 : 2) * slot + at, g);
+      spec_factor<M, true>(p2, mid, gz, d == 2, g);
+      row_c2r<M>(p2, ex, g, lane, tw);
+#pragma unroll
+      for (int j = 0; j < N1; ++j)
+        p2[j] = make_float2(__fmul_rn(c1, p2[j].x), __fmul_rn(c1, p2[j].y));
+    }
+#pragma unroll
+    for (int j = 0; j < N1; ++j)
+      p1[j] = make_float2(__fmul_rn(c0, p1[j].x), __fmul_rn(c0, p1[j].y));
+    const float q = d == 0 ? (float)(x - b * nx) : (float)(r - x * ny);
+#pragma unroll 1
+    for (int w = 0; w < 3; ++w) {  // disp, mom, force
+      float* st = stage[buf] + (lane / N2) * P + d;
+      const float f1 = w ? c[2 * w] : 1.f, f2 = w ? c[2 * w + 1] : 1.f;
+#pragma unroll
+      for (int j = 0; j < N1; ++j) {
+        const int k = 2 * (N2 * j + g);
+        float2 v = make_float2(__fmul_rn(f1, p1[j].x), __fmul_rn(f1, p1[j].y));
+        if (order == 2) {
+          v.x = __fadd_rn(v.x, __fmul_rn(f2, p2[j].x));
+          v.y = __fadd_rn(v.y, __fmul_rn(f2, p2[j].y));
+        }
+        if (w == 0 && shift) {
+          v.x = __fadd_rn(v.x, d == 2 ? (float)k : q);
+          v.y = __fadd_rn(v.y, d == 2 ? (float)(k + 1) : q);
+        }
+        // lanes alternate between the two cells: odd and even banks
+        st[3 * k + 3 * (g & 1)] = g & 1 ? v.y : v.x;
+        st[3 * k + 3 - 3 * (g & 1)] = g & 1 ? v.x : v.y;
+      }
+      __syncthreads();
+      float4* o = reinterpret_cast<float4*>(w == 0 ? disp : w == 1 ? mom
+                                                                   : force) +
+                  (size_t)r0 * (3 * NZ / 4);
+      // the block leaves this buffer alone until the barrier after next
+#pragma unroll 4
+      for (int e = threadIdx.x; e < RW * (3 * NZ / 4); e += kLptOutThreads) {
+        const int row = e / (3 * NZ / 4), t = e - row * (3 * NZ / 4);
+        o[e] = *reinterpret_cast<const float4*>(stage[buf] + row * P + 4 * t);
+      }
+      buf ^= 1;
+    }
+  }
+}
+
 // Output modes of k_fft_plane_inv.
 enum PlaneOut {
   kOutStencil = 0,  // potential -> phi, force y and z by the 4-point stencil
@@ -1240,6 +1632,116 @@ void launch_fft_zy_inv(const SimDev* sims, int first, int n, int nx, int ny,
                              : k_fft_z_inv<128, false>);
   k<<<z_grid(nx, ny, M, n), kZThreads, 0, st>>>(sims, first, nx * ny, spec,
                                                 phi, fmesh, nsteps, pos);
+}
+
+// ---------------------------------------------------------------------------
+// 2LPT passes
+// ---------------------------------------------------------------------------
+bool lpt_fused_supported(int nx, int ny, int nz) {
+  const auto ok = [](int n) {
+    return n >= 16 && n <= 512 && (n & (n - 1)) == 0;
+  };
+  return ok(nx) && ok(ny) && ok(nz);
+}
+
+namespace {
+
+#define FPM_LPT_SIZES(X) X(16) X(32) X(64) X(128) X(256) X(512)
+#define FPM_LPT_HALF(X) X(8) X(16) X(32) X(64) X(128) X(256)
+
+int row_blocks(int nrows, int M, int threads, int per_sm) {
+  int n2 = 2;  // Split<M>::N2
+  if (M >= 16) n2 = 4;
+  if (M >= 64) n2 = 8;
+  if (M >= 256) n2 = 16;
+  const int per = threads / n2, blocks = (nrows + per - 1) / per;
+  return blocks < kNumSMs * per_sm ? blocks : kNumSMs * per_sm;
+}
+
+}  // namespace
+
+int lpt_fused_prepare() {
+  if (prepare_device() != FPM_OK) return FPM_ERR_CUDA;
+  for (const void* k :
+       {(const void*)k_lpt_x<512>, (const void*)k_lpt_y_fwd<512>,
+        (const void*)k_lpt_y_inv<512>})
+    if (allow_smem(k, x_smem<512>()) != FPM_OK) return FPM_ERR_CUDA;
+  return FPM_OK;
+}
+
+void launch_lpt_fused(const LptRun& R, cudaStream_t st) {
+  g_launches.fetch_add(R.order == 2 ? 9 : 5, std::memory_order_relaxed);
+  const int M = R.nz / 2, nrows = R.count * R.nx * R.ny;
+  const unsigned nzh = M + 4;  // lpt_pitch
+  const int64_t slot = (int64_t)nrows * nzh;
+  const unsigned ygrid = (unsigned)((int64_t)R.count * R.nx * nzh / kXCols);
+  const int nblk = (int)(R.ny * nzh / kXCols);
+  const float* gy = R.grad + R.nx;
+  const float* gz = gy + R.ny;
+  float2 *u = R.six, *t = R.four, *sp = t + 3 * slot;
+  switch (M) {
+#define FPM_LPT_ROWS(MM)                                                  \
+  case MM:                                                                \
+    k_lpt_rows_fwd<MM><<<row_blocks(nrows, MM, kLptZThreads, 16),         \
+                         kLptZThreads, 0, st>>>(R.linear, sp, nrows); \
+    break;
+    FPM_LPT_HALF(FPM_LPT_ROWS)
+#undef FPM_LPT_ROWS
+  }
+  for (int pass = 1; pass <= R.order; ++pass) {
+    const int nout = pass == 1 && R.order == 2 ? 3 : 2;
+    const LptSlots S = nout == 3   ? LptSlots{{0, 1, 2, 3, 4, 5}}
+                       : pass == 1 ? LptSlots{{0, 1, 3}}
+                                   : LptSlots{{2, 4, 5}};
+    switch (R.ny) {
+#define FPM_LPT_Y(N)                                                     \
+  case N:                                                                \
+    k_lpt_y_fwd<N><<<ygrid, x_threads<N>(), x_smem<N>(), st>>>(sp, nzh); \
+    break;
+      FPM_LPT_SIZES(FPM_LPT_Y)
+#undef FPM_LPT_Y
+    }
+    switch (R.nx) {
+#define FPM_LPT_X(N)                                                         \
+  case N:                                                                    \
+    k_lpt_x<N><<<(unsigned)(R.count * nblk), x_threads<N>(), x_smem<N>(),    \
+                 st>>>(sp, t, slot, nblk, R.ny, nzh, R.kk2, R.grad, nout); \
+    break;
+      FPM_LPT_SIZES(FPM_LPT_X)
+#undef FPM_LPT_X
+    }
+    switch (R.ny) {
+#define FPM_LPT_Y(N)                                                       \
+  case N:                                                                  \
+    k_lpt_y_inv<N><<<ygrid, x_threads<N>(), x_smem<N>(), st>>>(t, u, slot, \
+                                                               nzh, gy, nout, S); \
+    break;
+      FPM_LPT_SIZES(FPM_LPT_Y)
+#undef FPM_LPT_Y
+    }
+    if (pass == 1 && R.order == 2) {
+      switch (M) {
+#define FPM_LPT_ROWS(MM)                                                  \
+  case MM:                                                                \
+    k_lpt_rows_source<MM><<<row_blocks(nrows, MM, kLptZThreads, 12),      \
+                            kLptZThreads, 0, st>>>(u, slot, sp, nrows, gz); \
+    break;
+        FPM_LPT_HALF(FPM_LPT_ROWS)
+#undef FPM_LPT_ROWS
+      }
+    }
+  }
+  switch (M) {
+#define FPM_LPT_ROWS(MM)                                                   \
+  case MM:                                                                 \
+    k_lpt_rows_out<MM><<<row_blocks(nrows, MM, 32, 16), kLptOutThreads, 0, \
+                         st>>>(                                            \
+        u, slot, R.order, gz, R.coef, nrows, R.nx, R.ny, R.shift, R.disp,  \
+        R.mom, R.force);                                                   \
+    break;
+    FPM_LPT_HALF(FPM_LPT_ROWS)
+#undef FPM_LPT_ROWS
+  }
 }
 
 }  // namespace fpm

@@ -130,6 +130,22 @@ void launch_fft_xpass(const SimDev* sims, int first, int n, int nx, int ny,
 // plain mesh; zero: clears what it reads.  Inverse: in place on spec, then
 // C2R along z into phi and, with fmesh, the z component of the 4-point
 // gradient into the third plane of each sim.
+// 2LPT of a run of equal lattices (pointers at its first simulation): linear
+// field -> disp (positions with shift), mom, force, each
+// count * nx * ny * nz * 3 floats (all 16-byte aligned).  six and four: scratch of
+// 6 and 4 times nx * ny * (nz / 2 + 4) modes per simulation.  kk2, grad: the lattice's axis
+// tables; coef: six per simulation.
+struct LptRun {
+  int count, nx, ny, nz, order, shift;
+  const float* linear;
+  float2 *six, *four;
+  const float2* kk2;
+  const float *grad, *coef;
+  float *disp, *mom, *force;
+};
+bool lpt_fused_supported(int nx, int ny, int nz);
+int lpt_fused_prepare();
+void launch_lpt_fused(const LptRun& R, cudaStream_t st);
 bool fft_zy_supported(int ny, int nz);
 void launch_fft_zy_fwd(const SimDev* sims, int first, int n, int nx, int ny,
                        int nz, float* rho, bool painted, bool pairs, int zero,

@@ -45,6 +45,7 @@ struct Run {
                            // around the x-pass kernel
   bool zy = false;         // x pass with the library's own z and y passes
                            // (r2c / c2r1 unused)
+  bool lpt = false;        // fused 2LPT passes (lr2c, lc2r9, lc2r3 unused there)
   int div_xc = 0;          // x chunk of the tiled divergence stencil
   // Simulations of the run still active at leapfrog position it (a prefix
   // when the run is ordered by non-increasing step count), and the batched
@@ -895,6 +896,13 @@ extern "C" int fpm_plan_create(fpm_plan** out, int nsims, const int32_t* dims,
       r.xpass = true;
       r.zy = fft_zy_supported(S0.my, S0.mz);
       for (int s = r.first; s < r.first + r.count; ++s) p->sims[s].xpass = 1;
+    }
+  }
+  if (lpt && !(flags & FPM_PLAN_CUFFT)) {
+    for (auto& r : p->runs) {
+      const SimDev& S0 = p->sims[r.first];
+      r.lpt = lpt_fused_supported(S0.nx, S0.ny, S0.nz) &&
+              lpt_fused_prepare() == FPM_OK;
     }
   }
   p->all_xpass = !p->runs.empty();
@@ -2005,9 +2013,23 @@ extern "C" int fpm_nbody_set_tape(fpm_plan* p, float* tape, int64_t floats) {
   return FPM_OK;
 }
 
-extern "C" int fpm_lpt_init(fpm_plan* p, const float* linear,
-                            const double* coef, int order, float* disp,
-                            float* mom, float* force, void* stream) {
+namespace {
+
+// Whether every run takes the fused passes with these arrays (rows are
+// accessed as float2 and float4).
+bool lpt_fused(const fpm_plan* p, const float* linear, const float* disp,
+               const float* mom, const float* force) {
+  for (const void* a : {(const void*)linear, (const void*)disp,
+                        (const void*)mom, (const void*)force})
+    if ((uintptr_t)a % 16 != 0) return false;
+  for (auto& r : p->runs)
+    if (!r.lpt) return false;
+  return true;
+}
+
+// fpm_lpt_init; with shift, disp holds positions.
+int lpt_init(fpm_plan* p, const float* linear, const double* coef, int order,
+             int shift, float* disp, float* mom, float* force, void* stream) {
   const Use use(p, (cudaStream_t)stream);
   if (!p || !linear || !coef || !disp || !mom || !force ||
       (order != 1 && order != 2))
@@ -2018,6 +2040,26 @@ extern "C" int fpm_lpt_init(fpm_plan* p, const float* linear,
   for (size_t i = 0; i < c.size(); ++i) c[i] = (float)coef[i];
   FPM_CUDA(cudaMemcpyAsync(p->d_lcoef, c.data(), sizeof(float) * c.size(),
                            cudaMemcpyHostToDevice, st));
+  if (lpt_fused(p, linear, disp, mom, force)) {
+    const AxisTabs tabs = tabs_of(p);
+    for (auto& r : p->runs) {
+      const SimDev& S = p->sims[r.first];
+      LptRun R = {r.count, S.nx, S.ny, S.nz, order, shift};
+      R.linear = linear + S.l_off;
+      // nine half spectra, nine lattice meshes: nz >= 16
+      R.six = p->lspec9 + 9 * S.ls_off;
+      R.four = reinterpret_cast<float2*>(p->lreal9 + 9 * S.l_off);
+      R.kk2 = tabs.kk2 + S.ltab;
+      R.grad = tabs.grad + S.ltab;
+      R.coef = p->d_lcoef + 6 * r.first;
+      R.disp = disp + 3 * S.p_off;
+      R.mom = mom + 3 * S.p_off;
+      R.force = force + 3 * S.p_off;
+      launch_lpt_fused(R, st);
+    }
+    FPM_TRY(launch_ok());
+    return settle(p, st);
+  }
   // cuFFT R2C may use its input as scratch for some sizes: transform a copy.
   FPM_CUDA(cudaMemcpyAsync(p->lreal1, linear, sizeof(float) * p->total_l,
                            cudaMemcpyDeviceToDevice, st));
@@ -2054,7 +2096,28 @@ extern "C" int fpm_lpt_init(fpm_plan* p, const float* linear,
   launch_lpt_particles(p->d_sims, p->nsims, p->ch_p, p->lreal9, 9, psi2, 3,
                        p->d_lcoef, disp, mom, force, st);
   FPM_TRY(launch_ok());
+  if (shift) {
+    for (auto& r : p->runs) {
+      const SimDev& S = p->sims[r.first];
+      FPM_TRY(fpm_lattice_shift(disp + 3 * S.p_off, disp + 3 * S.p_off,
+                                r.count, S.nx, S.ny, S.nz, 1, st));
+    }
+  }
   return settle(p, st);
+}
+
+}  // namespace
+
+extern "C" int fpm_lpt_init(fpm_plan* p, const float* linear,
+                            const double* coef, int order, float* disp,
+                            float* mom, float* force, void* stream) {
+  return lpt_init(p, linear, coef, order, 0, disp, mom, force, stream);
+}
+
+extern "C" int fpm_lpt_state(fpm_plan* p, const float* linear,
+                             const double* coef, int order, float* pos,
+                             float* mom, float* force, void* stream) {
+  return lpt_init(p, linear, coef, order, 1, pos, mom, force, stream);
 }
 
 extern "C" int fpm_lpt1(fpm_plan* p, const void* dlin_kv, const float* pos,

@@ -190,11 +190,9 @@ def lpt_init(cosmo, linear, a, order=2, kvec=None, name='LPTInit'):
   coef = np.tile(bg.lpt_coefficients(cosmo, a), B)
   state = torch.empty((3, B, np_, 3), dtype=torch.float32, device=linear.device)
   st = _lib.stream_ptr()
-  _lib.call('fpm_lpt_init', plan.handle, _lib.ptr(linear), _lib.dvec(coef),
+  _lib.call('fpm_lpt_state', plan.handle, _lib.ptr(linear), _lib.dvec(coef),
             order, _lib.ptr(state[0]), _lib.ptr(state[1]), _lib.ptr(state[2]),
             st)
-  _lib.call('fpm_lattice_shift', _lib.ptr(state[0]), _lib.ptr(state[0]), B,
-            nx, ny, nz, 1, st)
   return state
 
 

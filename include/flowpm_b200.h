@@ -158,7 +158,7 @@ int fpm_plan_info(const fpm_plan* plan, int64_t* total_particles,
                   int64_t* device_bytes);
 /* With enable, the plan's calls that are noted to synchronise the stream
  * (fpm_nbody_set_steps, fpm_nbody_set_pgd, fpm_pgd, fpm_lpt_init,
- * fpm_lpt_adjoint) are stream-ordered only, and the plan's calls and graph
+ * fpm_lpt_state, fpm_lpt_adjoint) are stream-ordered only, and the plan's calls and graph
  * launches on different streams run one after the other; fpm_plan_status
  * still synchronises.  Off for a new plan. */
 int fpm_plan_set_async(fpm_plan* plan, int enable);
@@ -371,6 +371,10 @@ int fpm_nbody_set_tape(fpm_plan* plan, float* tape, int64_t floats);
 int fpm_lpt_init(fpm_plan* plan, const float* linear, const double* coef,
                  int order, float* disp, float* mom, float* force,
                  void* stream);
+/* The same with positions pos = d + lattice point (fpm_lattice_shift). */
+int fpm_lpt_state(fpm_plan* plan, const float* linear, const double* coef,
+                  int order, float* pos, float* mom, float* force,
+                  void* stream);
 
 /* First-order LPT displacement read out at arbitrary positions,
  * flowpm/tfpm.py:66-95 lpt1: for each simulation s of the plan,
