@@ -282,6 +282,11 @@ def drift(cosmo, state, ai, ac, af, name='Drift', **kwargs):
   return state
 
 
+# nbody runs of at least this many particles work in their output (2^24: the
+# smallest of a few milliseconds a step).
+_DIRECT_PARTICLES = 1 << 24
+
+
 def nbody(cosmo, state, stages, nc, pm_nc_factor=1,
           return_intermediate_states=False, pgdparams=None, name='NBody',
           check_finite=True, checkpoint_every=None, store_potential=None):
@@ -339,10 +344,19 @@ def nbody(cosmo, state, stages, nc, pm_nc_factor=1,
   _lib.call('fpm_nbody_set_pgd', plan.handle, 0 if par is None else 1,
             None if par is None else _lib.dvec(np.tile(par, (B, 1)).ravel()),
             st)
-  d, p, f = plan.work()
+  # A large run works in its output, without the captured graph (a launch is
+  # nothing beside its kernels) and the copies to and from its buffers: 512^3,
+  # 6 steps: 35.0 -> 33.9 ms (B200).  16-byte aligned, as the buffers are.
+  direct = (T > 0 and plan.total_particles >= _DIRECT_PARTICLES and
+            plan.total_particles % 4 == 0 and not return_intermediate_states)
+  if direct:
+    out = torch.empty_like(state)
+    d, p, f = out[0], out[1], out[2]
+  else:
+    d, p, f = plan.work()
   _lib.call('fpm_lattice_shift', _lib.ptr(state[0]), _lib.ptr(d), B, nc[0],
             nc[1], nc[2], -1, st)
-  p.copy_(state[1].reshape(-1, 3))
+  p.copy_(state[1].reshape(p.shape))
   if par is None:
     tune(plan, d, p, (T, False))
   inter = None
@@ -352,12 +366,18 @@ def nbody(cosmo, state, stages, nc, pm_nc_factor=1,
     _lib.call('fpm_nbody_run', plan.handle, _lib.ptr(d), _lib.ptr(p),
               _lib.ptr(f), _lib.ptr(inter), _lib.FPM_NBODY_INTERMEDIATE, None,
               0, st)
+  elif direct:
+    _lib.call('fpm_nbody_run', plan.handle, _lib.ptr(d), _lib.ptr(p),
+              _lib.ptr(f), None, 0, None, 0, st)
   else:
     plan.launch_nbody(T, st)
-  out = torch.empty_like(state)
-  _to_pos(d.reshape(state[0].shape), nc, out[0])
-  out[1].copy_(p.reshape(state[1].shape))
-  out[2].copy_(f.reshape(state[2].shape))
+  if direct:
+    _to_pos(out[0], nc, out[0])
+  else:
+    out = torch.empty_like(state)
+    _to_pos(d.reshape(state[0].shape), nc, out[0])
+    out[1].copy_(p.reshape(state[1].shape))
+    out[2].copy_(f.reshape(state[2].shape))
   if check_finite:
     status = plan.status(st)
     if status:
