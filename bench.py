@@ -865,8 +865,10 @@ def measure_large(fpm, flush, reps=2, n=512, steps=30, ckpt=5, tape=True):
   # 12 Np + 4 Nc; the Fourier solve (density -> three force meshes, all of
   # its transforms and kernels) reads and zeroes the density and writes the
   # three force meshes, 20 Nc; its Green's-function kernel reads and writes
-  # the half spectrum (8 B per mode each) and zeroes the density, its
-  # stencil reads the potential and writes the three force meshes.
+  # the half spectrum (8 B per mode each), its stencil reads the potential
+  # and writes the three force meshes; on meshes of 256 or 512 the row passes
+  # along z clear the density and take the z component, elsewhere these two
+  # kernels do.
   # Reverse sweep, per particle (Np = Nc): the drift + paint kernel reads
   # d, F and reads and writes lam_x, p, lam_p (12 B each way), writes d,
   # gathers the adjoint density and paints (4 B per cell each), 116 B (112 B
@@ -883,8 +885,8 @@ def measure_large(fpm, flush, reps=2, n=512, steps=30, ckpt=5, tape=True):
       'step': KERNEL_BYTES_PER_PART * tot_np,
       'paint': 12 * tot_np + 4 * nc_tot,
       'fourier': 20 * nc_tot,
-      'green': 16 * half + 4 * nc_tot,
-      'stencil': 16 * nc_tot,
+      'green': 16 * half + (0 if n in (256, 512) else 4) * nc_tot,
+      'stencil': (12 if n in (256, 512) else 16) * nc_tot,
       # with the potential tape the reverse drift does not paint
       'adj_drift_paint': (112 if tape else 116) * tot_np,
       'adj_vjp': 112 * tot_np,

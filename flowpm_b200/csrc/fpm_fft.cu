@@ -14,13 +14,17 @@
 //       inverse DFT along y, complex-to-real along z, y and z components of
 //       the force by the stencil; k_fft_stencil_x takes the x component.
 //
+// Meshes of 256 or 512 take each axis as its own pass (k_fft_z_fwd, k_fft_y,
+// k_fft_x, k_fft_z_inv), and the 2LPT of power-of-two lattices passes shared by
+// its outputs (k_lpt_*).
+//
 // The transforms are unnormalised in both directions, as cuFFT's, so the
 // spectra have cuFFT's R2C layout (x, y, z/2 + 1) and the results match
 // the cuFFT path to rounding.  Every length-N DFT runs as N = N1 * N2 (the
 // "four-step" split): a group of N2 threads, each holding N1 values in
 // registers, does N1-point DFTs, a twiddle, one exchange through shared
-// memory and N2-point DFTs.  Twiddles come from a table of
-// exp(-2 pi i m / 128) computed in double on the host.
+// memory and N2-point DFTs.  Twiddles come from tables of exp(-2 pi i m / 128)
+// and exp(-2 pi i m / 512) computed in double on the host.
 #include <cmath>
 #include <mutex>
 

@@ -1,7 +1,5 @@
 """Binned power spectrum mirroring ``flowpm/pk.py`` (``power_spectrum``),
 computed on the device by the C library (fpm_power_spectrum)."""
-import ctypes
-
 import numpy as np
 import torch
 
@@ -36,13 +34,13 @@ def power_spectrum(field, kmin=5, dk=0.5, boxsize=False):
   out = torch.empty((B, len(kedges) - 1), dtype=torch.float32,
                     device=field.device)
   # scratch from torch's allocator: an allocation of the library's own would
-  # go back to the driver at every synchronisation
-  nbytes = ctypes.c_int64()
-  _lib.call('fpm_power_spectrum_work', B, nx, ny, nz, len(kedges),
-            ctypes.byref(nbytes))
-  work = torch.empty(nbytes.value, dtype=torch.uint8, device=field.device)
+  # go back to the driver at every synchronisation; the size is that of
+  # fpm_power_spectrum_work (spectrum, then the sums and weights of the bins)
+  nbytes = (-(-8 * B * nx * ny * (nz // 2 + 1) // 16) * 16 +
+            16 * B * (len(kedges) + 1))
+  work = torch.empty(nbytes, dtype=torch.uint8, device=field.device)
   _lib.call('fpm_power_spectrum_ws', _lib.ptr(field), B, nx, ny, nz,
             _lib.dvec(boxsize), float(kmin), float(dk), len(kedges),
-            _lib.ptr(out), _lib.ptr(work), nbytes.value, _lib.stream_ptr())
+            _lib.ptr(out), _lib.ptr(work), nbytes, _lib.stream_ptr())
   kbins = kedges[:-1] + (kedges[1:] - kedges[:-1]) / 2
   return kbins, out
